@@ -133,7 +133,7 @@ alt2_kernel(const ResArgs a) {
     __shared__ unsigned int s_alive[3];          // float form: images alive after layer li % 3
     __shared__ int s_ns[3];                      // float form: layer li % 3 produced an output that is neither 0 nor clip
     __shared__ unsigned int s_grp[2][2];         // bit form, many warps: {unsaturated, last layer's outputs} of a group
-    __shared__ int s_x[4];                       // state handed from the bit form to the block
+    __shared__ int s_x[5];                       // state handed from the bit form to the block
     __shared__ int s_last, s_fail;
     __shared__ int s_next_group;                 // the next group of tables to request (used by one thread at a time)
     __shared__ __align__(8) unsigned long long s_bar[kAlt2MaxTableRing];
@@ -272,6 +272,7 @@ alt2_kernel(const ResArgs a) {
         // ---- the layers of this chunk
         int li = 0;                  // layers of the chunk applied so far
         int last_classes = 0;
+        int nl = a.nlayers;          // layers to apply (a fixed point of the bit form moves it forward)
         const bool force_dead = a.bias > 0.0f;
         const bool multi = a.bit_multi != 0;     // layers of more than one pass of 64 classes: all warps work in the bit form
         // Otherwise ONE warp of the block does the bit form.  Warp w of every block sits on the same scheduler
@@ -287,7 +288,7 @@ alt2_kernel(const ResArgs a) {
             __syncthreads();
             bitmode = true;
         }
-        while (li < a.nlayers) {
+        while (li < nl) {
             if (bitmode) {
                 // ---- bit form.  Worker warps (one warp when a layer is one pass of 64 classes, else
                 //      all warps) apply groups of layers until the chunk ends, every image is dead, or a
@@ -301,7 +302,8 @@ alt2_kernel(const ResArgs a) {
                     int waited_group = -1;                   // the group of tables these threads have seen arrive
                     unsigned int tt_cur = 0xffffffffu;       // no truth table has this value
                     TruthMasks tm = truth_masks(0u);
-                    while (li < a.nlayers) {
+                    bool first_period = true;                // the first periodic group is one period, so that a fixed point shows early
+                    while (li < nl) {
                         if (STAGED && (li >> gshift) != waited_group) {
                             if (leader) issue_groups(li);
                             const bool arrived = wait_table(li);
@@ -312,9 +314,15 @@ alt2_kernel(const ResArgs a) {
                             }
                             waited_group = li >> gshift;
                         }
-                        int cnt = min(a.wring - 1, a.nlayers - li);
+                        int cnt = min(a.wring - 1, nl - li);
                         if (STAGED) cnt = min(cnt, (1 << gshift) - (li & gmask));
                         if (careful > 0) cnt = 1;
+                        // whole periods of the chunk's tables where one fits (see below: fixed point)
+                        bool periodic = a.period > 0 && li >= a.period_from && cnt >= a.period;
+                        if (periodic) {
+                            cnt = first_period ? a.period : cnt / a.period * a.period;
+                            first_period = false;
+                        }
                         const unsigned char *T = table_of(li);
                         // The layers of a group are applied with one truth table: lane g looks at layer g's, and
                         // a group whose layers differ (another K or weight) is cut down to its first layer.
@@ -323,7 +331,7 @@ alt2_kernel(const ResArgs a) {
                             const unsigned int tl = STAGED ? *reinterpret_cast<const unsigned int *>(hp) : __ldg(reinterpret_cast<const unsigned int *>(hp));
                             const unsigned int t0 = __shfl_sync(0xffffffffu, tl, 0);
                             const bool same = multi ? __syncthreads_and(tl == t0 ? 1 : 0) != 0 : __all_sync(0xffffffffu, tl == t0);
-                            if (!same) cnt = 1;
+                            if (!same) { cnt = 1; periodic = false; }
                             if (t0 != tt_cur) {
                                 tt_cur = t0;
                                 tm = truth_masks(t0);
@@ -422,14 +430,26 @@ alt2_kernel(const ResArgs a) {
                         }
                         if (now != alive && leader) atomicAdd(a.died_at + li, __popc(alive & ~now));     // cnt == 1
                         alive = now;
-                        ws = s;
                         li += cnt;
                         done_classes = classes;
+                        if (periodic && li < nl) {
+                            // Fixed point: the tables repeat with this period and the group's last words are those it
+                            // started from (its first buffer is still intact), so every later whole period changes
+                            // nothing -- no image dies in one and no output is unsaturated, as none was in this one --
+                            // and only the layers behind the last whole period are left.  They use the tables of the
+                            // layers that follow here.  (1024 neurons, layers 41 .. 1919 of 60000 images: 239 -> 15 us.)
+                            const unsigned int *w0 = wring0 + (size_t)ws * a.rows_w, *w1 = wring0 + (size_t)s * a.rows_w;
+                            unsigned int moved = 0u;
+                            for (int q = multi ? tid : lane; q < classes; q += multi ? NT : 32) moved |= w0[q] ^ w1[q];
+                            if (multi ? !__syncthreads_or(moved != 0u ? 1 : 0) : __all_sync(0xffffffffu, moved == 0u))
+                                nl = li + (nl - li) % a.period;
+                        }
+                        ws = s;
                         if (careful > 0) --careful;
                         if (alive == 0u) break;
                     }
                     if (leader) {
-                        s_x[0] = li; s_x[1] = (int)alive; s_x[2] = done_classes; s_x[3] = ws;
+                        s_x[0] = li; s_x[1] = (int)alive; s_x[2] = done_classes; s_x[3] = ws; s_x[4] = nl;
                         s_alive[li % 3] = 0u;        // the float form may take over at layer li
                         s_ns[li % 3] = 0;
                     }
@@ -439,6 +459,7 @@ alt2_kernel(const ResArgs a) {
                 alive_prev = (unsigned int)s_x[1];
                 last_classes = s_x[2];
                 ws = s_x[3];
+                nl = s_x[4];
                 // back to floats: the rows the next float layer (or the expansion below) reads
                 const unsigned int *wcur = wring0 + (size_t)ws * a.rows_w;
                 for (int r = grp; r < a.buf_rows; r += CPI) {
@@ -532,7 +553,7 @@ alt2_kernel(const ResArgs a) {
                 alive_prev = 0u;
             }
             if (alive_prev == 0u) break;
-            if (saturated && li < a.nlayers) {
+            if (saturated && li < nl) {
                 // every output of the layer is 0 or clip: continue in the bit form
                 wring0 = reinterpret_cast<unsigned int *>(nxt);
                 rows_to_bits(cur, wring0);

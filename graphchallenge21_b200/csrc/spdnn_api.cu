@@ -142,6 +142,7 @@ struct spdnn {
     bool bits_small = false;           // SPDNN_BITS_SMALL=1: the pre-pass also for chunks whose layers have at most 64 classes
                                        // (one warp per 32 images)
     bool table_cache = true;           // SPDNN_TABLE_CACHE=0: the pre-pass always streams its layer records
+    bool fixed_point = true;           // SPDNN_FIXED_POINT=0: the bit forms apply every period of a periodic network
     bool two_blocks = true;            // SPDNN_TWO_BLOCKS=0: ALT2 chunks keep the largest group of images per block even where it leaves one block per SM
     int alt2_threads = 0;              // SPDNN_ALT2_THREADS=256|512: block size of ALT2 chunks with 4 images per thread (0: by shared memory)
     int bits_threads = 0;              // SPDNN_BITS_THREADS: threads per block of the pre-pass (0: by the classes)
@@ -509,7 +510,23 @@ struct Step {
     unsigned char *cache = nullptr;
     unsigned short *rec_of = nullptr;
     int cache_records = 0;
+    int period = 0, period_from = 0;      // ALT2 chunk: its tables repeat with this period from this layer of the chunk on (0: no)
 };
+
+// Period of an ALT2 chunk's tables: the smallest P such that the chunk ends in at least two periods of layers whose
+// tables (matrix and value ids) repeat with P, and the first layer of that part.
+void find_period(spdnn *c, Step &st) {
+    constexpr int kMaxPeriod = 31;        // the bit forms check at most 31 or 32 layers at once
+    for (int p = 1; p <= kMaxPeriod && 2 * p <= st.count; ++p) {
+        int q = st.count - p;             // layers [q, count - p) equal those p further on
+        while (q > 0 && c->res[st.first + q - 1] == c->res[st.first + q - 1 + p]) --q;
+        if (st.count - q >= 2 * p) {
+            st.period = p;
+            st.period_from = q;
+            return;
+        }
+    }
+}
 
 // The launches of one pass, front to back.
 // dense_first: the pass starts from the caller's row-major input; its first launch is then a resident
@@ -521,6 +538,7 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
     int resident_chunks = 0;       // resident chunks planned so far
     int alt2_chunks = 0;           // ALT2 chunks planned so far
     int generic_chunks = 0;        // GENERIC chunks planned so far
+    int short_chunk = 0;           // > 0: `chunk` was raised to the rest of the network at once; the length it would have had
     while (l < c->layers) {
         Step st;
         st.first = l;
@@ -576,6 +594,8 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                     // on its way while one is applied, as many word buffers as a group has layers plus the one
                     // it starts from -- whatever of that fits
                     st.max_classes = maxc;
+                    st.count = f;
+                    if (c->fixed_point && c->bit_form) find_period(c, st);
                     st.stride = alt2_stream_stride(maxc);
                     st.rows_w = std::max(rows, 32);
                     // staging may take a quarter of the shared memory at most, so that the blocks per SM stay
@@ -593,6 +613,12 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                         return alt2_smem_bytes(t_i, rows, st.stride, st.gshift, st.tring);
                     };
                     const size_t need = stage(ti, (size_t)c->smem_optin);
+                    if (short_chunk > 0 && !(st.period > 0 && st.period < st.wring)) {
+                        // no fixed point to look for, or no room to look for it: grow step by step (see below)
+                        chunk = short_chunk;
+                        short_chunk = 0;
+                        continue;
+                    }
                     // A block that has an SM to itself cannot hide the loading and storing of its rows, nor the tail of a
                     // layer, behind another block's arithmetic: where half the images per block (and tables staged at
                     // least four layers at a time) let two blocks share an SM, that is faster (measured at 16384 neurons).
@@ -651,15 +677,29 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
         if (st.ti) {
             ++resident_chunks;
             if (resident_chunks < (int)c->chunk_list.size()) chunk = c->chunk_list[resident_chunks];
-            // A chunk with a bits_kernel pre-pass runs its saturated tiles at a fraction of the float form's cost and
-            // dead images cost it nothing, so such chunks can be long.  But a tile that is NOT saturated when the chunk
-            // starts is the float form's for the whole chunk (at 65536 neurons about 1.4 us per layer and tile against
-            // 0.3): the first chunk with a pre-pass is as short as the chunk before it, and only the one after it takes
-            // the rest of the network -- a tile that saturates a few layers late then costs tens of layers, not
-            // thousands (measured: one such tile among 7500 images made a pass 2.6 ms longer).
-            else if ((st.max_classes > 64 || c->bits_small) && st.max_classes > 0 && alt2_chunks >= 1 && c->bits_prepass && c->bit_form && c->clip > 0.0f && !c->chunk_growth_set)
-                chunk = alt2_chunks >= 2 ? c->chunk_max : chunk;
-            else chunk = std::min(chunk * (st.max_classes > 0 ? c->chunk_growth : c->chunk_growth_generic), c->chunk_max);
+            else {
+                const bool alt2 = st.max_classes > 0;
+                const bool prepass = alt2 && (st.max_classes > 64 || c->bits_small) && c->bits_prepass && c->bit_form && c->clip > 0.0f;
+                short_chunk = 0;
+                if (prepass && alt2_chunks >= 1 && !c->chunk_growth_set) {
+                    // A chunk with a bits_kernel pre-pass runs its saturated tiles at a fraction of the float form's cost
+                    // and dead images cost it nothing, so such chunks can be long.  But a tile that is NOT saturated when
+                    // the chunk starts is alt2_kernel's for the whole chunk (at 65536 neurons about 1.4 us per layer and
+                    // tile against 0.3): the first chunk with a pre-pass is as short as the chunk before it, and only the
+                    // one after it takes the rest of the network -- a tile that saturates a few layers late then costs
+                    // tens of layers, not thousands (measured: one such tile among 7500 images made a pass 2.6 ms longer).
+                    if (alt2_chunks >= 2) chunk = c->chunk_max;
+                } else {
+                    chunk = std::min(chunk * (alt2 ? c->chunk_growth : c->chunk_growth_generic), c->chunk_max);
+                }
+                // Where the tables repeat, alt2_kernel's own bit form ends a tile one period after it saturates
+                // (ResArgs::period): from the third ALT2 chunk on one launch takes the rest of the network, provided that
+                // its word ring has room for a period (checked when the chunk is planned).
+                if (alt2 && alt2_chunks == 1 && c->fixed_point && c->bit_form && !c->chunk_growth_set && chunk < c->chunk_max) {
+                    short_chunk = chunk;
+                    chunk = c->chunk_max;
+                }
+            }
         }
         if (st.ti && st.max_classes > 0) ++alt2_chunks;
         if (st.ti && st.max_classes == 0) ++generic_chunks;
@@ -738,6 +778,7 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
             a.bit_ok = (alt2 && c->bit_form && c->clip > 0.0f && st.wring >= 2) ? 1 : 0;
             a.tile_done = nullptr; a.wwords = 0;
             a.cache = nullptr; a.rec_of = nullptr; a.cache_records = 0;
+            a.period = st.period; a.period_from = st.period_from;
             a.gate = nullptr; a.gate_want = 0;
             if (alt2 && st.bits_threads > 0) {
                 // pre-pass: tiles of 32 images that are saturated already run the whole chunk as words
@@ -1065,6 +1106,7 @@ int spdnn_create(spdnn_t **out, int device, int neurons, int layers, float bias,
         if (const char *e = getenv("SPDNN_COUNT_FRONT")) c->count_front = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_BITS_KERNEL")) c->bits_prepass = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_BITS_FIRST")) c->bits_first_chunk = atoi(e) != 0;
+        if (const char *e = getenv("SPDNN_FIXED_POINT")) c->fixed_point = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_TWO_BLOCKS")) c->two_blocks = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_TABLE_CACHE")) c->table_cache = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_BITS_SMALL")) c->bits_small = atoi(e) != 0;

@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) bits_kernel(const ResArgs 
     TruthMasks tm = truth_masks(0u);
     unsigned int ns = 0u;
     int li = 0, last_classes = 0;
+    int nl = a.nlayers;                              // layers still to be applied end here (a fixed point moves it forward)
     int waited_group = -1;
     bool failed = false, unsat = false;
     auto run_tracked = [&](int lend) {
@@ -238,8 +239,24 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) bits_kernel(const ResArgs 
             auto entries = [&](const unsigned char *rec, int ps) -> uint2 {
                 return ps < spasses ? (reinterpret_cast<const uint2 *>(rec + 16 + ps * 256))[lane] : make_uint2(0u, 0u);
             };
-            while (li < a.nlayers && !unsat && !failed) {
-                const int l0 = li, l1 = min(li + kBitsCheckEvery, a.nlayers);
+            // Fixed point: where the chunk's tables repeat with period P, a segment is whole periods, and a segment that
+            // ends in the words it started from (every row of every image) has shown that all later periods do the same:
+            // only what is left behind the last whole period has to be applied.  The challenge networks get there one
+            // period after they saturate, so a tile costs tens of layers instead of thousands (layers 41 .. 1919 at 16384
+            // neurons: 490 tiles 617 -> 60 us, two tiles, where nothing hides the chain's latency, 371 -> 71 us; at 65536
+            // neurons 235 tiles 682 -> 148 us; what is left loads and stores the tiles' rows).
+            const int period = a.period > 0 && a.period <= kBitsCheckEvery ? a.period : 0;
+            int seg = period;                                       // the first periodic segment is one period, later ones as many as fit
+            while (li < nl && !unsat && !failed) {
+                const int l0 = li;
+                const bool periodic = period > 0 && li >= a.period_from && li + period <= nl;
+                int l1 = min(li + kBitsCheckEvery, nl);
+                if (periodic) {
+                    l1 = li + (li + seg <= nl ? seg : period);
+                    seg = kBitsCheckEvery / period * period;
+                } else if (period > 0 && li < a.period_from) {
+                    l1 = min(l1, a.period_from);
+                }
                 for (int q = tid; q < a.wwords; q += blockDim.x) ckpt[q] = wc[q];      // read before layer l0's barrier, which precedes any write to wc
                 const unsigned char *T = tbl0 + (size_t)s_rec[li] * stride;
                 int classes = *reinterpret_cast<const int *>(T);
@@ -260,7 +277,7 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) bits_kernel(const ResArgs 
                     const unsigned int b4 = *reinterpret_cast<const unsigned int *>(wcb + (e1.y >> 16));
                     const bool has0 = p0 < passes, has1 = p1 < passes;
                     last_classes = classes;
-                    if (li + 1 < a.nlayers) {                       // the next layer's record, while the words arrive
+                    if (li + 1 < nl) {                              // the next layer's record, while the words arrive
                         const unsigned char *Tn = tbl0 + (size_t)s_rec[li + 1] * stride;
                         classes = *reinterpret_cast<const int *>(Tn);
                         e0 = entries(Tn, p0);
@@ -280,15 +297,19 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) bits_kernel(const ResArgs 
                     unsigned int *t = wc; wc = wn; wn = t;
                 }
                 // who is alive after the segment: the OR of the last layer's rows
-                unsigned int o = 0u;
-                for (int q = tid; q < last_classes; q += blockDim.x) o |= wc[q];
+                unsigned int o = 0u, moved = 0u;
+                for (int q = tid; q < last_classes; q += blockDim.x) {
+                    o |= wc[q];
+                    moved |= wc[q] ^ ckpt[q];
+                }
                 o = __reduce_or_sync(0xffffffffu, o);
                 if (lane == 0 && o) atomicOr(&s_or[0], o);
                 const bool any_ns = __syncthreads_or(nsx != 0u ? 1 : 0) != 0;      // (the barrier also publishes the atomics)
                 const unsigned int now = s_or[0] & alive;
-                __syncthreads();                               // everyone has read s_or[0]
+                const bool fixed = !__syncthreads_or(moved != 0u ? 1 : 0) && periodic;      // (everyone has read s_or[0])
                 if (tid == 0) s_or[0] = s_or[1] = s_or[2] = 0u;
                 if (any_ns) { unsat = true; break; }
+                if (fixed) nl = li + (nl - li) % period;       // (nobody died: a dead image's words were not all zero before)
                 if (now != alive) {
                     // somebody died inside the segment: again from its input, layer by layer (the tracked loop wants
                     // its three slots zero and leaves them in any state)
@@ -302,10 +323,10 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) bits_kernel(const ResArgs 
                 if (alive == 0u) break;
             }
         } else {
-            run_tracked(a.nlayers);
+            run_tracked(nl);
         }
     } else {
-        run_tracked(a.nlayers);
+        run_tracked(nl);
     }
     if (STAGED) {
         if (tid == 0) drain(li);

@@ -101,6 +101,9 @@ struct ResArgs {
     const unsigned char *cache;
     const unsigned short *rec_of;
     int cache_records;
+    // The chunk's tables repeat: layer q + period uses the tables of layer q for every q >= period_from (0: no period).
+    // Saturated activations that one period maps onto themselves are then a fixed point of all later periods.
+    int period, period_from;
     // the launch runs only when *gate == gate_want (nullptr: always), see LayerArgs
     const int32_t *gate;
     int gate_want;
