@@ -117,6 +117,23 @@ inline std::string canonicalize_layer(int n, const int32_t *col_ptr, const int32
     return std::string();
 }
 
+// Whether the layer maps the vector whose every entry is `clip` onto itself: each column's sum, added and rounded as the
+// kernels do it, reaches clip with the bias.  (Every product and sum is rounded to fp32 by its store.)
+inline bool keeps_top(const HostLayer &h, float bias, float clip) {
+    for (int c = 0; c < h.n; ++c) {
+        const int32_t *r = &h.rows[(size_t)c * h.k];
+        volatile float sum = 0.0f;
+        for (int i = 0; i < h.k && r[i] < h.n; ++i) {
+            volatile float term = h.uniform ? clip : clip * h.vals[(size_t)c * h.k + i];
+            sum = sum + term;
+        }
+        volatile float y = h.uniform ? sum * h.w : sum;
+        y = y + bias;
+        if (!(y >= clip)) return false;
+    }
+    return true;
+}
+
 // Groups the columns of a layer whose (id sequence, weights) coincide.  ids == nullptr: the
 // sequences are the raw rows.  Classes are numbered in order of their first column.
 inline int group_columns(const HostLayer &h, const int32_t *ids, std::vector<int> &class_of, std::vector<int> &first_col) {

@@ -631,6 +631,8 @@ alt2_kernel(const ResArgs a) {
     la.first_member_only = 0;
     la.bias = a.bias; la.clip = a.clip;
     la.xw = nullptr; la.nw = 0; la.gate = nullptr; la.gate_want = 0;
+    la.retire = a.retire;
+    la.retire.open = nullptr;
     rebuild_worklist(la, live_in, ctl.ids_buf);
 }
 

@@ -39,6 +39,7 @@ struct DevLayer {
     int32_t *mem = nullptr;
     int classes = 0, k = 0;
     bool uniform = false, identity_members = false;
+    bool keeps_top = false;               // maps the all-clip vector onto itself
     float w = 0.0f;
     int64_t nnz = 0;
     uint64_t h1 = 0, h2 = 0;
@@ -131,6 +132,13 @@ struct spdnn {
     // Binary inputs (spdnn_front.cuh): the input as one word per (tile, neuron); in_flag is raised on the device
     // while an input is converted when it holds a value other than 0 and 1, and picks the variant of the first
     // layer's launches; has_floats marks the tiles whose float form was written.
+    uint32_t *open_mask = nullptr;        // [tiles] ballots of images with an activation that is not clip (struct Retire)
+    uint32_t *settled = nullptr, *working = nullptr;      // [tiles] bitmaps over image numbers: retired, still on the work list
+    int32_t *work_of = nullptr;           // [images] position of a survivor in the work list, -1: retired
+    int32_t *first_cell = nullptr;        // global number of the batch's first image
+    bool retire = true;                // SPDNN_RETIRE=0: all-clip images stay on the work list
+    int settle_from = 0;               // from this layer on every layer maps the all-clip vector onto itself
+    bool retires = false;              // a launch of the captured schedule retires images
     uint32_t *xw = nullptr;
     int nw = 0;
     int32_t *in_flag = nullptr;
@@ -149,7 +157,7 @@ struct spdnn {
     int extra_launches = 0;            // pre-pass launches of the captured schedule
     int graph_extra[2] = {0, 0};
     int32_t *ids[2] = {nullptr, nullptr};
-    unsigned int *counter = nullptr;   // [0] blocks finished, [1] next work item
+    unsigned int *counter = nullptr;   // [0] blocks finished, [1] next work item, [2] images retired by a launch
     int32_t *status = nullptr;
 
     void *stage = nullptr;             // device staging for host inputs / outputs
@@ -206,6 +214,8 @@ int fail(spdnn *c, int code, const char *fmt, ...) {
 int free_buffers(spdnn *c) {
     cudaFree(c->y[0]); cudaFree(c->y[1]); cudaFree(c->slot); cudaFree(c->mask); cudaFree(c->tile_done);
     cudaFree(c->ids[0]); cudaFree(c->ids[1]); cudaFree(c->xw); cudaFree(c->has_floats);
+    cudaFree(c->open_mask); cudaFree(c->settled); cudaFree(c->working); cudaFree(c->work_of);
+    c->open_mask = c->settled = c->working = nullptr; c->work_of = nullptr;
     c->y[0] = c->y[1] = nullptr; c->slot = nullptr; c->mask = nullptr; c->ids[0] = c->ids[1] = nullptr;
     c->tile_done = nullptr; c->xw = nullptr; c->has_floats = nullptr;
     c->tiles_cap = 0;
@@ -226,6 +236,11 @@ int ensure_capacity(spdnn *c, int batch) {
     CK(cudaMalloc(&c->slot, sizeof(int32_t) * (size_t)tiles * 32));
     CK(cudaMalloc(&c->mask, sizeof(uint32_t) * (size_t)tiles));
     CK(cudaMemsetAsync(c->mask, 0, sizeof(uint32_t) * (size_t)tiles, c->stream));
+    CK(cudaMalloc(&c->open_mask, sizeof(uint32_t) * (size_t)tiles));
+    CK(cudaMemsetAsync(c->open_mask, 0, sizeof(uint32_t) * (size_t)tiles, c->stream));
+    CK(cudaMalloc(&c->settled, sizeof(uint32_t) * (size_t)tiles));
+    CK(cudaMalloc(&c->working, sizeof(uint32_t) * (size_t)tiles));
+    CK(cudaMalloc(&c->work_of, sizeof(int32_t) * (size_t)tiles * 32));
     CK(cudaMalloc(&c->tile_done, (size_t)tiles));
     CK(cudaMemsetAsync(c->tile_done, 0, (size_t)tiles, c->stream));
     CK(cudaMalloc(&c->xw, sizeof(uint32_t) * (size_t)tiles * c->nw));
@@ -286,7 +301,7 @@ int repair_float_tiles(spdnn *c) {
 
 int end_input(spdnn *c) {
     init_loop_kernel<<<std::max(1, std::min(1024, (c->batch + 255) / 256)), 256, 0, c->stream>>>(
-        c->ctl, c->ids[0], c->batch, c->first_id, c->died_at, c->layers, c->dense_cell, c->dense_src);
+        c->ctl, c->ids[0], c->batch, c->first_id, c->died_at, c->layers, c->dense_cell, c->dense_src, c->first_cell, c->settled, c->working, c->tiles_cap);
     CK(cudaGetLastError());
     c->prep_launches += 1;
     CK(cudaEventRecord(c->ev_prep1, c->stream));
@@ -691,6 +706,14 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                     if (alt2_chunks >= 2) chunk = c->chunk_max;
                 } else {
                     chunk = std::min(chunk * (alt2 ? c->chunk_growth : c->chunk_growth_generic), c->chunk_max);
+                    // Images without structure saturate one by one soon after the first chunk, at clip everywhere, and leave the
+                    // list at the end of a chunk: chunks of 2, 2, 4, 8, ... layers follow the first one (59 % of the survivors are gone at
+                    // layer 8 of such a network of 1024 neurons, 89 % at 10, 96 % at 12; with 16 layers after the first 8 the float form
+                    // ran them all for everyone: 3866 us for 60000 images, in the short chunks 640).
+                    if (!alt2 && c->retire && !c->chunk_growth_set && l + st.count >= c->settle_from) {
+                        if (generic_chunks == 0) chunk = std::min(chunk, 2);
+                        else if (generic_chunks == 1) chunk = std::min(chunk, 2);
+                    }
                 }
                 // Where the tables repeat, alt2_kernel's own bit form ends a tile one period after it saturates
                 // (ResArgs::period): from the third ALT2 chunk on one launch takes the rest of the network, provided that
@@ -727,6 +750,7 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
     c->last_group = 0;
     c->extra_launches = 0;
     c->streamed_launches = 0;
+    c->retires = false;
     int front = kFrontNone;
     if (gated) {
         if (plan[0].ti == 0) {
@@ -755,6 +779,13 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
         const bool lazy_last = c->lazy_expand && c->reps_only && step + 1 == plan.size() && st.ti != 0 && c->res[last_layer] &&
                                c->res[last_layer]->mem_ptr != nullptr;
         if (step + 1 == plan.size()) c->expand_layer_of_plan = lazy_last ? last_layer : -1;
+        // (the last launch has nothing behind it to spare; the variants of layer 0 on binary inputs do not look for clip; saturated
+        // tiles of an ALT2 chunk cost one period of its tables, less than the bookkeeping here)
+        Retire retire;
+        retire.open = c->open_mask; retire.settled = c->settled; retire.first_id = c->first_cell;
+        retire.count = c->counter + 2;
+        retire.on = c->retire && !(st.ti && c->res[l]->mode == kResAlt2) && step + 1 < plan.size() && last_layer + 1 >= c->settle_from && !(step == 0 && front == kFrontWords) ? 1 : 0;
+        if (retire.on) c->retires = true;
         if (st.ti) {
             const DevRes &R0 = *c->res[l];
             ResArgs a;
@@ -780,6 +811,8 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
             a.cache = nullptr; a.rec_of = nullptr; a.cache_records = 0;
             a.period = st.period; a.period_from = st.period_from;
             a.gate = nullptr; a.gate_want = 0;
+            a.retire = retire;
+            a.settle_from = c->retire ? std::max(0, c->settle_from - l) : st.count + 1;
             if (alt2 && st.bits_threads > 0) {
                 // pre-pass: tiles of 32 images that are saturated already run the whole chunk as words
                 ResArgs b = a;                 // (gated like the launch it prepares)
@@ -883,6 +916,8 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
             a.first_member_only = (next_reads_reps && !L.identity_members) ? 1 : 0;
             a.bias = c->bias; a.clip = c->clip;
             a.xw = nullptr; a.nw = 0; a.gate = nullptr; a.gate_want = 0;
+            a.retire = retire;
+            a.retire.count = nullptr;
             const long long ncb = (L.classes + d.classes_per_item - 1) / d.classes_per_item;
             if ((long long)c->tiles_cap * ncb >= 0xffffffffLL) return fail(c, SPDNN_ERR_LIMIT, "batch too large for one launch");
             int grid = c->grid_override > 0 ? c->grid_override : c->sm_count * blocks_per_sm(L.k, L.uniform);
@@ -920,8 +955,14 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
     }
     c->nsteps = (int)plan.size();
     finalize_ids_kernel<<<std::max(1, std::min(c->tiles_cap, 4 * c->sm_count)), 256, 0, c->stream>>>(c->ctl + c->nsteps, c->slot,
-                                                                                             c->ids[0], c->ids[1]);
+                                                                                             c->ids[0], c->ids[1], c->working, c->first_cell);
     CK(cudaGetLastError());
+    if (c->retires) {
+        merge_settled_kernel<<<(c->tiles_cap + kMergeWords - 1) / kMergeWords, 256, 0, c->stream>>>(c->ctl + c->nsteps, c->ids[0], c->ids[1], c->working, c->settled, c->tiles_cap,
+                                                        c->first_cell, c->work_of);
+        CK(cudaGetLastError());
+        c->extra_launches += 1;
+    }
     return SPDNN_OK;
 }
 
@@ -995,6 +1036,8 @@ int build_graph(spdnn *c) {
     c->streams.clear();
     int rc = prepare_resident(c);
     if (rc) return rc;
+    c->settle_from = c->layers;
+    while (c->settle_from > 0 && c->layer[c->settle_from - 1]->keeps_top) --c->settle_from;
     {
         // device slots of the streamed layers: two, each as large as the largest of them
         size_t need = 0;
@@ -1073,9 +1116,10 @@ int spdnn_create(spdnn_t **out, int device, int neurons, int layers, float bias,
     c->layer.resize(layers);
     CK(cudaMalloc(&c->ctl, sizeof(LoopCtl) * (size_t)(layers + 1)));
     CK(cudaMemset(c->ctl, 0, sizeof(LoopCtl) * (size_t)(layers + 1)));
-    CK(cudaMalloc(&c->counter, 2 * sizeof(unsigned int)));
-    CK(cudaMemset(c->counter, 0, 2 * sizeof(unsigned int)));
+    CK(cudaMalloc(&c->counter, 3 * sizeof(unsigned int)));
+    CK(cudaMemset(c->counter, 0, 3 * sizeof(unsigned int)));
     CK(cudaMalloc(&c->status, sizeof(int32_t)));
+    CK(cudaMalloc(&c->first_cell, sizeof(int32_t)));
     CK(cudaMalloc(&c->dense_cell, sizeof(const float *)));
     CK(cudaMemset(c->dense_cell, 0, sizeof(const float *)));
     CK(cudaMemset(c->status, 0, sizeof(int32_t)));
@@ -1106,6 +1150,7 @@ int spdnn_create(spdnn_t **out, int device, int neurons, int layers, float bias,
         if (const char *e = getenv("SPDNN_COUNT_FRONT")) c->count_front = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_BITS_KERNEL")) c->bits_prepass = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_BITS_FIRST")) c->bits_first_chunk = atoi(e) != 0;
+        if (const char *e = getenv("SPDNN_RETIRE")) c->retire = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_FIXED_POINT")) c->fixed_point = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_TWO_BLOCKS")) c->two_blocks = atoi(e) != 0;
         if (const char *e = getenv("SPDNN_TABLE_CACHE")) c->table_cache = atoi(e) != 0;
@@ -1147,7 +1192,7 @@ void spdnn_destroy(spdnn_t *c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (int kind = 0; kind < 2; ++kind)
         if (c->graph_exec[kind]) cudaGraphExecDestroy(c->graph_exec[kind]);
-    cudaFree(c->dense_cell);
+    cudaFree(c->dense_cell); cudaFree(c->first_cell);
     free_buffers(c);
     cudaFree(c->ctl); cudaFree(c->counter); cudaFree(c->status); cudaFree(c->stage); cudaFree(c->in_flag);
     cudaFree(c->died_at); cudaFree(c->res_table);
@@ -1214,6 +1259,7 @@ int spdnn_set_layer_csc(spdnn_t *c, int layer, const int32_t *col_ptr, const int
     auto L = std::make_shared<DevLayer>();
     L->device = c->device;
     L->classes = p.classes; L->k = host->k; L->uniform = host->uniform; L->identity_members = p.identity_members;
+    L->keeps_top = keeps_top(*host, c->bias, c->clip);
     L->w = host->w; L->nnz = host->nnz; L->h1 = host->hash1; L->h2 = host->hash2;
     const size_t table_bytes = 4 * (std::max<size_t>(p.off.size(), 4) + (host->uniform ? 0 : std::max<size_t>(p.vals.size(), 4)) +
                                     p.mem_ptr.size() + std::max<size_t>(p.mem.size(), 1));
@@ -1515,7 +1561,7 @@ int spdnn_sync(spdnn_t *c, spdnn_stats_t *stats) {
         }
         spdnn_stats_t s{};
         s.layers = c->layers; s.batch = c->batch;
-        s.survivors = c->host_ctl[c->nsteps].live;
+        s.survivors = c->host_ctl[c->nsteps].live + c->host_ctl[c->nsteps].settled;
         {
             long long live = c->batch;
             for (int l = 0; l < c->layers; ++l) {
@@ -1566,11 +1612,12 @@ int spdnn_get_categories(spdnn_t *c, int32_t *ids, int capacity, int *count) {
     if (c->in_flight) { int rc = spdnn_sync(c, nullptr); if (rc) return rc; }
     if (!c->result_ready) return fail(c, SPDNN_ERR_STATE, "no result: call spdnn_infer first");
     const LoopCtl fin = c->host_ctl[c->nsteps];
-    *count = fin.live;
-    if (fin.live == 0) return SPDNN_OK;
-    if (!ids || capacity < fin.live) return fail(c, SPDNN_ERR_ARG, "capacity %d < survivors %d", capacity, fin.live);
+    const int total = fin.live + fin.settled;
+    *count = total;
+    if (total == 0) return SPDNN_OK;
+    if (!ids || capacity < total) return fail(c, SPDNN_ERR_ARG, "capacity %d < survivors %d", capacity, total);
     DeviceGuard guard(c->device);
-    CK(cudaMemcpyAsync(ids, c->ids[fin.ids_buf], sizeof(int32_t) * (size_t)fin.live, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(ids, c->ids[fin.settled ? fin.ids_buf ^ 1 : fin.ids_buf], sizeof(int32_t) * (size_t)total, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return SPDNN_OK;
 }
@@ -1579,7 +1626,8 @@ int spdnn_get_activations(spdnn_t *c, float *y, int64_t capacity_rows) {
     if (!c) return SPDNN_ERR_ARG;
     if (c->in_flight) { int rc = spdnn_sync(c, nullptr); if (rc) return rc; }
     if (!c->result_ready) return fail(c, SPDNN_ERR_STATE, "no result: call spdnn_infer first");
-    const int live = c->host_ctl[c->nsteps].live;
+    const LoopCtl fin_ctl = c->host_ctl[c->nsteps];
+    const int live = fin_ctl.live + fin_ctl.settled;
     if (live == 0) return SPDNN_OK;
     if (!y || capacity_rows < live) return fail(c, SPDNN_ERR_ARG, "capacity %lld < survivors %d", (long long)capacity_rows, live);
     DeviceGuard guard(c->device);
@@ -1605,7 +1653,7 @@ int spdnn_get_activations(spdnn_t *c, float *y, int64_t capacity_rows) {
         const size_t rows = std::min(chunk_rows, (size_t)live - r0);
         const dim3 block(32, 8), grid((unsigned)((rows + 31) / 32), (c->n + 31) / 32);
         tiles_to_dense_kernel<<<grid, block, 0, c->stream>>>(fin, c->tile_stride, c->ctl + c->nsteps, c->slot, c->n,
-                                                            (float *)c->stage, (int)r0);
+                                                            (float *)c->stage, (int)r0, fin_ctl.settled ? c->work_of : nullptr, c->clip);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(y + r0 * c->n, c->stage, rows * row_bytes, cudaMemcpyDeviceToHost, c->stream));
     }

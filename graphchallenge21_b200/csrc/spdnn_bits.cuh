@@ -412,6 +412,8 @@ __device__ __forceinline__ unsigned int planes_ge(const unsigned int (&p)[6], in
 __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned int s_or[3];
+    __shared__ unsigned int s_open[3];           // images with an output of layer li % 3 that is not clip
+    __shared__ volatile int s_float;             // a value that is neither 0 nor clip was seen
     __shared__ int s_nev, s_ev_layer[32], s_ev_cnt[32];
     __shared__ float s_tab[64];                  // output of the current layer for every count 0 .. K
     if (a.gate != nullptr && *a.gate != a.gate_want) return;
@@ -431,7 +433,10 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
     const float *__restrict__ p = a.yin + (size_t)(src >> 5) * a.tile_stride + (src & 31);
     const ResLayer L0 = a.layers[0];
     bool ns_in = false;
-    for (int v0 = warp * 8; v0 < L0.v_in; v0 += nwarps * 8) {
+    unsigned int not_all = 0u;
+    if (tid == 0) s_float = 0;
+    __syncthreads();
+    for (int v0 = warp * 8; v0 < L0.v_in && !__any_sync(0xffffffffu, s_float); v0 += nwarps * 8) {       // (most tiles of the early chunks are the float form's: stop reading)
         int e[8];
         float x[8];
 #pragma unroll
@@ -445,14 +450,16 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
         for (int q = 0; q < 8; ++q) {
             const unsigned int w = __ballot_sync(0xffffffffu, x[q] != 0.0f);
             ns_in |= (x[q] != 0.0f && x[q] != a.clip);
+            not_all |= ~w;
             if (lane == 0 && v0 + q < L0.v_in) wc[resident_phys_row(v0 + q)] = w;
         }
+        if (__any_sync(0xffffffffu, ns_in) && lane == 0) s_float = 1;
     }
     // every word past the value ids is zero in both buffers: padded table entries point at the first even row behind them
     for (int r = L0.v_in + tid; r < a.wwords; r += blockDim.x) wc[(r < ((L0.v_in + 1) & ~1)) ? resident_phys_row(r) : r] = 0u;
     for (int r = tid; r < a.wwords; r += blockDim.x) wn[r] = 0u;
     if (tid == 0) {
-        s_or[0] = 0u;
+        s_or[0] = s_open[0] = 0u;
         s_nev = 0;
     }
     if (__syncthreads_or(ns_in ? 1 : 0)) {
@@ -465,9 +472,12 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
     unsigned int ns = 0u;
     int li = 0, last_classes = 0;
     bool unsat = false;
+    // every image alive is all clip and every layer to come keeps that: nothing is left to apply
+    bool settled = a.settle_from <= 0 && !__syncthreads_or((not_all & alive) != 0u ? 1 : 0);
+    unsigned int open_now = settled ? 0u : 0xffffffffu;
     int tab_k = -1, sat_lo = 0, zero_hi = 0;
     float tab_w = 0.0f;
-    while (li < a.nlayers) {
+    while (li < a.nlayers && !settled) {
         const ResLayer RL = a.layers[li];
         const int classes = RL.classes, k = RL.k;
         if (k != tab_k || RL.w != tab_w) {
@@ -496,7 +506,7 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
         const int passes = (classes + 31) >> 5;
         const int kp = k + 4;
         const int32_t *__restrict__ tb = RL.blob + 4;
-        unsigned int o = 0u;
+        unsigned int o = 0u, open = 0u;
         for (int ps = warp; ps < passes; ps += nwarps) {
             const int u = ps * 32 + lane;
             const bool in = u < classes;
@@ -529,6 +539,7 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
                 ns |= nz & ~x;
                 wn[resident_phys_row(u)] = x;
                 o |= x;
+                open |= ~x;
             }
         }
         {
@@ -538,10 +549,13 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
             for (int r = classes + tid; r < ue + 2; r += blockDim.x) wn[r < ue ? resident_phys_row(r) : r] = 0u;
         }
         o = __reduce_or_sync(0xffffffffu, o);
+        open = __reduce_or_sync(0xffffffffu, open);
         if (lane == 0 && o) atomicOr(&s_or[li % 3], o);
-        if (tid == 0) s_or[(li + 1) % 3] = 0u;
+        if (lane == 0 && open) atomicOr(&s_open[li % 3], open);
+        if (tid == 0) s_or[(li + 1) % 3] = s_open[(li + 1) % 3] = 0u;
         __syncthreads();
         const unsigned int now = s_or[li % 3] & alive;
+        open_now = s_open[li % 3];
         if (now != alive && tid == 0) {
             s_ev_layer[s_nev] = li;
             s_ev_cnt[s_nev] = __popc(alive & ~now);
@@ -551,7 +565,8 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
         unsigned int *t = wc; wc = wn; wn = t;
         last_classes = classes;
         ++li;
-        if ((li % kBitsCheckEvery) == 0 || li == a.nlayers || alive == 0u) {
+        settled = (alive & open_now) == 0u && li >= a.settle_from;
+        if ((li % kBitsCheckEvery) == 0 || li == a.nlayers || alive == 0u || settled) {
             if (__syncthreads_or(ns != 0u ? 1 : 0)) { unsat = true; break; }
         }
         if (alive == 0u) break;
@@ -560,12 +575,21 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) count_kernel(const ResArgs
         if (tid == 0) a.tile_done[tile] = 0;
         return;
     }
+    const unsigned int top = a.retire.on ? alive & ~open_now : 0u;      // images that have reached their result leave the work list
     if (tid == 0) {
         a.tile_done[tile] = 1;
         for (int q = 0; q < s_nev; ++q) atomicAdd(a.died_at + s_ev_layer[q], s_ev_cnt[q]);
-        if (alive) atomicOr(a.mask + tile, alive);
+        if (alive & ~top) atomicOr(a.mask + tile, alive & ~top);
+        if (top) atomicAdd(a.retire.count, (unsigned int)__popc(top));
     }
-    if (alive == 0u) return;
+    if (warp == 0 && top != 0u) retire_images(a.retire, ctl.ids_buf ? a.ids1 : a.ids0, tile * 32, top);
+    if ((alive & ~top) == 0u) return;
+    if (settled && li < a.nlayers) {
+        li = a.nlayers;
+        last_classes = a.layers[li - 1].classes;
+        for (int u = tid; u < last_classes; u += blockDim.x) wc[resident_phys_row(u)] = alive;
+        __syncthreads();
+    }
     const ResLayer LL = a.layers[li - 1];
     float *out = a.yout + (size_t)tile * a.tile_stride + lane;
     for (int u = warp; u < last_classes; u += nwarps) {

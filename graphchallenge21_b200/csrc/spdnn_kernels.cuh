@@ -46,8 +46,30 @@ struct LoopCtl {
     int32_t live;        // images alive
     int32_t identity;    // 1: image j sits in slot j of the input buffer (no indirection)
     int32_t ids_buf;     // which of the two id arrays holds the ids in current order
-    int32_t reserved;
+    int32_t settled;     // images retired so far because every activation was clip and stays so (not among `live`)
 };
+
+// Images whose activations are all clip at a layer boundary behind which every layer maps that vector onto itself
+// (checked on the weights when the network is set) have reached their result: they leave the work list as the dead
+// images do, marked in a bitmap, and join the survivors after the last launch (merge_settled_kernel).  Where weights have no
+// structure that is every survivor, a few layers after the first chunk (us a pass, before -> after: 60000 images, 1024
+// neurons, 120 layers 10900 -> 4804; 3000 images, 16384 neurons, 24 layers, one launch per layer, 7947 -> 4143).
+struct Retire {
+    uint32_t *open;              // per-layer kernel: per output tile, ballot of lanes with an output other than clip (zero on entry and exit)
+    uint32_t *settled;           // bit (id - *first_id): image `id` was retired
+    const int32_t *first_id;
+    unsigned int *count;         // kernels whose blocks own whole images: images this launch retired (zero on entry and exit)
+    int on;                      // this launch retires: every later layer keeps the all-clip vector
+};
+
+// One warp, lane = image: marks the images j0 + (bits of top) as retired.  ids: the numbers in the order of this launch.
+__device__ __forceinline__ void retire_images(const Retire &r, const int32_t *ids, int j0, unsigned int top) {
+    const int lane = threadIdx.x & 31;
+    if ((top >> lane) & 1u) {
+        const int pos = __ldcg(ids + j0 + lane) - *r.first_id;
+        atomicOr(r.settled + (pos >> 5), 1u << (pos & 31));
+    }
+}
 
 struct LayerArgs {
     const float *yin;
@@ -72,6 +94,7 @@ struct LayerArgs {
     // for binary inputs and one for any input, and the flag raised while the input was converted picks one
     const int32_t *gate;
     int gate_want;
+    Retire retire;
 };
 
 // L2 residency hints of the per-layer kernel (SPDNN_L2_HINT: 0 none, 1 input rows are read
@@ -187,13 +210,32 @@ __device__ __forceinline__ float class_sum(const LayerDesc &d, int u, const floa
 // for the images they own (move_id), and finalize_ids_kernel does it after the last launch.
 __device__ __forceinline__ void rebuild_worklist(const LayerArgs &a, int live_in, int ids_buf) {
     __shared__ int s_warp[32];          // works for any block size up to 1024 threads
-    __shared__ int s_total;
+    __shared__ int s_total, s_settled;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ntiles = (live_in + 31) >> 5;
     const int nwarps = blockDim.x >> 5;
     const int per_warp = (ntiles + nwarps - 1) / nwarps;
     const int w0 = min(warp * per_warp, ntiles), w1 = min(w0 + per_warp, ntiles);
     int cnt = 0;
+    if (tid == 0) s_settled = a.retire.on && a.retire.count ? (int)__ldcg(a.retire.count) : 0;
+    __syncthreads();
+    if (a.retire.on && a.retire.open) {
+        // images that are done: note their numbers and take them off the list
+        int done = 0;
+        for (int tb = w0; tb < w1; tb += 32) {
+            const bool in = tb + lane < w1;
+            const uint32_t m = in ? __ldcg(a.mask + tb + lane) : 0u, top = in ? m & ~__ldcg(a.retire.open + tb + lane) : 0u;
+            if (in) a.retire.open[tb + lane] = 0u;
+            if (top) a.mask[tb + lane] = m & ~top;
+            done += __popc(top);
+            for (uint32_t some = __ballot_sync(0xffffffffu, top != 0u); some; some &= some - 1u) {
+                const int i = __ffs(some) - 1;
+                retire_images(a.retire, ids_buf ? a.ids1 : a.ids0, (tb + i) * 32, __shfl_sync(0xffffffffu, top, i));
+            }
+        }
+        if (done) atomicAdd(&s_settled, done);
+        __syncwarp();
+    }
     for (int t = w0 + lane; t < w1; t += 32) cnt += __popc(__ldcg(a.mask + t));
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, d);      // survivors of the warp's run
@@ -210,8 +252,8 @@ __device__ __forceinline__ void rebuild_worklist(const LayerArgs &a, int live_in
         if (lane == nwarps - 1) s_total = w;
     }
     __syncthreads();
-    const int total = s_total;
-    if (total > live_in && tid == 0) atomicExch(a.status, 2);
+    const int total = s_total, settled = s_settled;
+    if (total + settled > live_in && tid == 0) atomicExch(a.status, 2);
     const bool same = (total == live_in);      // nobody died: positions are already dense
     if (!same) {
         int run = warp ? s_warp[warp - 1] : 0;         // first position of this warp's run
@@ -233,11 +275,12 @@ __device__ __forceinline__ void rebuild_worklist(const LayerArgs &a, int live_in
         c.live = total;
         c.identity = same ? 1 : 0;
         c.ids_buf = same ? ids_buf : (ids_buf ^ 1);
-        c.reserved = 0;
+        c.settled = a.ctl_in->settled + settled;
         *a.ctl_out = c;
         *a.counter = 0u;
         *a.work = 0u;
-        if (a.died_at) *a.died_at = live_in - total;
+        if (a.retire.on && a.retire.count) *a.retire.count = 0u;
+        if (a.died_at) *a.died_at = live_in - total - settled;
     }
 }
 
@@ -255,7 +298,7 @@ __device__ __forceinline__ void move_id(const LoopCtl &ctl, int32_t *ids0, int32
 // share input rows, and the second read of a row then hits in L1.
 template <int KT, bool UNIFORM, bool BITS = false>
 __global__ void __launch_bounds__(kThreads, SPDNN_MIN_BLOCKS) layer_kernel(const LayerDesc d, const LayerArgs a) {
-    __shared__ unsigned int s_mask;
+    __shared__ unsigned int s_mask, s_open;
     __shared__ unsigned int s_item;
     __shared__ int s_last;
     if (a.gate != nullptr && *a.gate != a.gate_want) return;
@@ -273,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, SPDNN_MIN_BLOCKS) layer_kernel(const
     for (;;) {
         if (tid == 0) {
             s_item = atomicAdd(a.work, 1u);
-            s_mask = 0u;
+            s_mask = s_open = 0u;
         }
         __syncthreads();
         const unsigned int item = s_item;
@@ -288,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, SPDNN_MIN_BLOCKS) layer_kernel(const
         const float *__restrict__ yin = BITS ? reinterpret_cast<const float *>(a.xw + (size_t)(src >> 5) * a.nw)
                                              : a.yin + (size_t)(src >> 5) * a.tile_stride + (src & 31);
         float *__restrict__ yout = a.yout + (size_t)tile * a.tile_stride + lane;
-        bool any = false;
+        bool any = false, open = false;
         const int u_end = min(d.classes, (cb + 1) * cpi);
         const int u0 = cb * cpi + warp * per_warp;
         const int u1 = min(u0 + per_warp, u_end);
@@ -304,6 +347,7 @@ __global__ void __launch_bounds__(kThreads, SPDNN_MIN_BLOCKS) layer_kernel(const
             const float s = class_sum<KT, UNIFORM, BITS>(d, u, yin, pol_in, src & 31);
             const float y = relu_clip(__fadd_rn(s, a.bias), a.clip);
             any |= (y != 0.0f);
+            open |= (y != a.clip);
             const int cnt = a.first_member_only ? 1 : me - mb;
             if (cnt <= 32) {
                 for (int m = 0; m < cnt; ++m) store_row(yout + __shfl_sync(0xffffffffu, mreg, m), y, pol_out);
@@ -313,8 +357,13 @@ __global__ void __launch_bounds__(kThreads, SPDNN_MIN_BLOCKS) layer_kernel(const
         }
         const unsigned int m = __ballot_sync(0xffffffffu, any && valid);
         if (lane == 0 && m) atomicOr(&s_mask, m);
+        if (a.retire.on) {
+            const unsigned int om = __ballot_sync(0xffffffffu, open && valid);
+            if (lane == 0 && om) atomicOr(&s_open, om);
+        }
         __syncthreads();
         if (tid == 0 && s_mask) atomicOr(a.mask + tile, s_mask);
+        if (tid == 0 && s_open) atomicOr(a.retire.open + tile, s_open);
     }
 
     // last block done: rebuild the work list (wait-free: nobody spins)
@@ -384,29 +433,75 @@ static __global__ void coo_to_tiles_kernel(const int32_t *__restrict__ img, cons
     }
 }
 
-// Tiles -> row-major [rows][N] for the live images j_base, j_base+1, ... in work-list order
-// (row 0 of `out` is image j_base).  Block (32, 8), grid (ceil(rows/32), ceil(N/32)).
+// Tiles -> row-major [rows][N] for the surviving images j_base, j_base+1, ... in ascending image number
+// (row 0 of `out` is image j_base).  Block (32, 8), grid (ceil(rows/32), ceil(N/32)).  work_of (nullptr: no image was
+// retired): position in the work list of survivor j, or -1 for a retired image, whose activations are all clip.
 static __global__ void tiles_to_dense_kernel(const float *__restrict__ y, long long tile_stride, const LoopCtl *ctl,
-                                      const int32_t *__restrict__ slot, int n, float *__restrict__ out, int j_base) {
+                                      const int32_t *__restrict__ slot, int n, float *__restrict__ out, int j_base,
+                                      const int32_t *__restrict__ work_of, float clip) {
     __shared__ float t[32][33];
     const LoopCtl c = *ctl;
+    const int total = c.live + c.settled;
     const int j0 = j_base + blockIdx.x * 32;
-    if (j0 >= c.live) return;
+    if (j0 >= total) return;
     const int c0 = blockIdx.y * 32;
     const int j = j0 + threadIdx.x;
-    const int jj = j < c.live ? j : j0;
-    const int src = c.identity ? jj : slot[jj];
+    const int jj = j < total ? j : j0;
+    const int k = work_of ? work_of[jj] : jj;
+    const int src = c.identity || k < 0 ? max(k, 0) : slot[k];
     const float *base = y + (size_t)(src >> 5) * tile_stride + (src & 31);
 #pragma unroll
     for (int r = threadIdx.y; r < 32; r += 8) {
         const int col = c0 + r;
-        t[r][threadIdx.x] = col < n ? base[(size_t)col * 32] : 0.0f;    // t[col][image]
+        t[r][threadIdx.x] = k < 0 ? clip : col < n ? base[(size_t)col * 32] : 0.0f;    // t[col][image]
     }
     __syncthreads();
 #pragma unroll
     for (int r = threadIdx.y; r < 32; r += 8) {
         const int img = j0 + r, col = c0 + threadIdx.x;
-        if (img < c.live && col < n) out[(size_t)(img - j_base) * n + col] = t[threadIdx.x][r];
+        if (img < total && col < n) out[(size_t)(img - j_base) * n + col] = t[threadIdx.x][r];
+    }
+}
+
+// After the last launch of a pass that retired images (finalize_ids_kernel marked the images still on the work list in
+// `working`): lists the survivors, working or retired, in ascending order into ids[ids_buf ^ 1], and notes for each its
+// position in the work list (-1: retired).  A block takes kMergeWords words of the bitmaps and counts all words before
+// them itself (a few KB from L2), so that blocks need not wait for one another.
+constexpr int kMergeWords = 64;
+static __global__ void __launch_bounds__(256) merge_settled_kernel(const LoopCtl *ctl, int32_t *ids0, int32_t *ids1, const uint32_t *__restrict__ working,
+                                                                   const uint32_t *__restrict__ settled, int words, const int32_t *first_id,
+                                                                   int32_t *work_of) {
+    __shared__ int s_all, s_work, s_cnt[2][kMergeWords];
+    const LoopCtl c = *ctl;
+    if (c.settled == 0) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = *first_id;
+    int32_t *to = c.ids_buf ? ids0 : ids1;
+    const int q0 = blockIdx.x * kMergeWords, q1 = min(q0 + kMergeWords, words);
+    if (tid == 0) s_all = s_work = 0;
+    __syncthreads();
+    int all = 0, work = 0;
+    for (int q = tid; q < q0; q += blockDim.x) {
+        const uint32_t w = working[q];
+        work += __popc(w);
+        all += __popc(w | settled[q]);
+    }
+    all = __reduce_add_sync(0xffffffffu, all);
+    work = __reduce_add_sync(0xffffffffu, work);
+    if (lane == 0) { atomicAdd(&s_all, all); atomicAdd(&s_work, work); }
+    if (q0 + tid < q1) {
+        s_cnt[0][tid] = __popc(working[q0 + tid] | settled[q0 + tid]);
+        s_cnt[1][tid] = __popc(working[q0 + tid]);
+    }
+    __syncthreads();
+    for (int q = q0 + warp; q < q1; q += (int)(blockDim.x >> 5)) {
+        int at = s_all, wat = s_work;
+        for (int p = 0; p < q - q0; ++p) { at += s_cnt[0][p]; wat += s_cnt[1][p]; }
+        const uint32_t w = working[q], m = w | settled[q], below = (1u << lane) - 1u;
+        if ((m >> lane) & 1u) {
+            const int j = at + __popc(m & below);
+            to[j] = first + q * 32 + lane;
+            work_of[j] = ((w >> lane) & 1u) ? wat + __popc(w & below) : -1;
+        }
     }
 }
 
@@ -427,24 +522,33 @@ static __global__ void expand_members_kernel(float *__restrict__ y, long long ti
     }
 }
 
-static __global__ void finalize_ids_kernel(const LoopCtl *ctl, const int32_t *__restrict__ slot, int32_t *ids0, int32_t *ids1) {
+static __global__ void finalize_ids_kernel(const LoopCtl *ctl, const int32_t *__restrict__ slot, int32_t *ids0, int32_t *ids1, uint32_t *working,
+                                           const int32_t *first_id) {
     const LoopCtl c = *ctl;
-    if (c.identity) return;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < c.live; j += gridDim.x * blockDim.x)
-        move_id(c, ids0, ids1, j, __ldg(slot + j));
+    if (c.identity && c.settled == 0) return;
+    int32_t *ids = c.ids_buf ? ids1 : ids0;
+    const int32_t *from = c.ids_buf ? ids0 : ids1;
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < c.live; j += gridDim.x * blockDim.x) {
+        const int32_t id = c.identity ? ids[j] : __ldg(from + __ldg(slot + j));
+        if (!c.identity) ids[j] = id;
+        if (c.settled) atomicOr(working + ((id - *first_id) >> 5), 1u << ((id - *first_id) & 31));
+    }
 }
 
 // dense_cell: where the first launch of a pass finds the caller's row-major input when that launch
 // reads it in place (dense_src, may be null: the input was converted to tiles).
 static __global__ void init_loop_kernel(LoopCtl *ctl, int32_t *ids0, int batch, int first_global_id, int32_t *died_at,
-                                        int layers, const float **dense_cell, const float *dense_src) {
+                                        int layers, const float **dense_cell, const float *dense_src, int32_t *first_cell,
+                                        uint32_t *settled, uint32_t *working, int words) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x)
         ids0[i] = first_global_id + i;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < layers; i += gridDim.x * blockDim.x) died_at[i] = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) settled[i] = working[i] = 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         LoopCtl c;
-        c.live = batch; c.identity = 1; c.ids_buf = 0; c.reserved = 0;
+        c.live = batch; c.identity = 1; c.ids_buf = 0; c.settled = 0;
         *ctl = c;
+        *first_cell = first_global_id;
         *dense_cell = dense_src;
     }
 }

@@ -107,6 +107,8 @@ struct ResArgs {
     // the launch runs only when *gate == gate_want (nullptr: always), see LayerArgs
     const int32_t *gate;
     int gate_want;
+    Retire retire;
+    int settle_from;          // from this layer of the chunk on to the end of the network every layer maps the all-clip vector onto itself
 };
 
 __host__ __device__ __forceinline__ int resident_phys_row(int r) {
@@ -353,6 +355,7 @@ resident_kernel(const ResArgs a) {
     constexpr int NT = SPDNN_GENERIC_THREADS;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned int s_alive[3];
+    __shared__ unsigned int s_open[3];           // images with an output of layer li % 3 that is not clip
     __shared__ int s_last, s_fail;
     __shared__ __align__(8) unsigned long long s_bar[2];
     if (a.gate != nullptr && *a.gate != a.gate_want) return;
@@ -375,7 +378,7 @@ resident_kernel(const ResArgs a) {
         unsigned char *const tbl0 = smem + 2 * buf_bytes;      // table buffer q sits at tbl0 + q * table_bytes
         const int j0 = blockIdx.x * TI;
         if (tid == 0) {
-            s_alive[0] = 0u;
+            s_alive[0] = s_open[0] = 0u;
             s_fail = 0;
             if (STAGED) {
                 mbar_init(&s_bar[0], 1);
@@ -447,13 +450,15 @@ resident_kernel(const ResArgs a) {
         }
         int li = 0;
         int last_classes = 0;
+        unsigned int open_now = 0xffffffffu;
+        bool settled = false;
         const bool force_dead = a.bias > 0.0f;
         for (; li < a.nlayers; ++li) {
             const int32_t *T;
             bool ready = true;
             if (STAGED) {
                 if (tid == 0) {
-                    s_alive[(li + 1) % 3] = 0u;
+                    s_alive[(li + 1) % 3] = s_open[(li + 1) % 3] = 0u;
                     // the other table buffer was last read in layer li - 1, which every thread has left
                     if (li + 1 < a.nlayers) {
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -468,7 +473,7 @@ resident_kernel(const ResArgs a) {
                 if (!ready) s_fail = 1;
                 T = reinterpret_cast<const int32_t *>(tbl0 + (li & 1) * a.table_bytes);
             } else {
-                if (tid == 0) s_alive[(li + 1) % 3] = 0u;
+                if (tid == 0) s_alive[(li + 1) % 3] = s_open[(li + 1) % 3] = 0u;
                 T = a.layers[li].blob;
             }
             // per-layer scalars travel in the table's header
@@ -477,7 +482,7 @@ resident_kernel(const ResArgs a) {
             const int classes = hdr.x, lk = hdr.y;
             const float lw = __int_as_float(hdr.z);
             last_classes = classes;
-            unsigned int bits = 0;
+            unsigned int bits = 0, open = 0;
             const unsigned char *in = cur + sub * TB;
             for (int u = grp; u < classes; u += CPI) {
                 float4 s[NQ];
@@ -505,6 +510,7 @@ resident_kernel(const ResArgs a) {
                         if (!(al & 8u)) y.w = 0.0f;
                     }
                     bits |= ((y.x != 0.0f ? 1u : 0u) | (y.y != 0.0f ? 2u : 0u) | (y.z != 0.0f ? 4u : 0u) | (y.w != 0.0f ? 8u : 0u)) << (4 * h);
+                    open |= ((y.x != a.clip ? 1u : 0u) | (y.y != a.clip ? 2u : 0u) | (y.z != a.clip ? 4u : 0u) | (y.w != a.clip ? 8u : 0u)) << (4 * h);
                     *reinterpret_cast<float4 *>(nxt + out_row * RS + sub * TB + 16 * h) = y;
                 }
             }
@@ -518,8 +524,11 @@ resident_kernel(const ResArgs a) {
             }
             const unsigned int wm = __reduce_or_sync(0xffffffffu, bits << (sub * IPT));
             if (lane == 0 && wm) atomicOr(&s_alive[li % 3], wm);
+            const unsigned int om = __reduce_or_sync(0xffffffffu, open << (sub * IPT));
+            if (lane == 0 && om) atomicOr(&s_open[li % 3], om);
             __syncthreads();
             const unsigned int alive_now = s_alive[li % 3] & alive_prev;
+            open_now = s_open[li % 3];
             if (tid == 0) {
                 const int died = __popc(alive_prev & ~alive_now);
                 if (died) atomicAdd(a.died_at + li, died);
@@ -531,6 +540,8 @@ resident_kernel(const ResArgs a) {
                 alive_prev = 0u;
             }
             if (alive_prev == 0u) { ++li; break; }
+            // every image still alive has reached its result: the rest of the chunk changes nothing
+            if ((alive_prev & open_now) == 0u && li + 1 >= a.settle_from && li + 1 < a.nlayers) { settled = true; ++li; break; }
         }
         if (STAGED && li < a.nlayers) {
             // the loop was left early with the table of layer li still on its way: wait for it
@@ -540,6 +551,21 @@ resident_kernel(const ResArgs a) {
             __syncthreads();
         }
 
+        if (settled && alive_prev != 0u) {
+            li = a.nlayers;
+            last_classes = a.layers[li - 1].classes;
+            const unsigned int al = alive_prev >> (sub * IPT);
+            for (int u = grp; u < last_classes; u += CPI)
+#pragma unroll
+                for (int h = 0; h < NQ; ++h)
+                    *reinterpret_cast<float4 *>(cur + resident_phys_row(u) * RS + sub * TB + 16 * h) =
+                        make_float4((al >> (4 * h)) & 1u ? a.clip : 0.0f, (al >> (4 * h)) & 2u ? a.clip : 0.0f,
+                                    (al >> (4 * h)) & 4u ? a.clip : 0.0f, (al >> (4 * h)) & 8u ? a.clip : 0.0f);
+            // (each thread stores below what it has just written itself)
+        }
+        // images that have reached their result leave the work list; what is left of the block's images is stored
+        const unsigned int top = a.retire.on ? alive_prev & ~open_now : 0u;
+        alive_prev &= ~top;
         // ---- expand the survivors' classes to all member rows (dead blocks write nothing)
         if (alive_prev != 0u) {
             const ResLayer LL = a.layers[li - 1];
@@ -581,6 +607,10 @@ resident_kernel(const ResArgs a) {
             }
             if (tid == 0) atomicOr(a.mask + tile, alive_prev << lane0);
         }
+        if (tid < 32 && top != 0u) {
+            retire_images(a.retire, ctl.ids_buf ? a.ids1 : a.ids0, j0, top);
+            if (tid == 0) atomicAdd(a.retire.count, (unsigned int)__popc(top));
+        }
     }
 
     // ---- last block done: rebuild the work list
@@ -600,6 +630,8 @@ resident_kernel(const ResArgs a) {
     la.first_member_only = 0;
     la.bias = a.bias; la.clip = a.clip;
     la.xw = nullptr; la.nw = 0; la.gate = nullptr; la.gate_want = 0;
+    la.retire = a.retire;
+    la.retire.open = nullptr;
     rebuild_worklist(la, live_in, ctl.ids_buf);
 }
 

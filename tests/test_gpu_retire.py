@@ -1,0 +1,54 @@
+"""GPU tests of retired images (every activation clip, every later layer keeps that): same bits as the oracle, which
+applies every layer to every image."""
+import numpy as np
+import pytest
+
+from conftest import mixed_density_images, rows_of
+from graphchallenge21_b200 import SpDNN
+from graphchallenge21_b200.generator import SyntheticNetwork, synthetic_images
+
+pytestmark = pytest.mark.gpu
+
+
+def run(n, layers, bias, clip, y0, first):
+    with SpDNN(n, len(layers), bias, clip=clip) as g:
+        for l, (rows, vals) in enumerate(layers):
+            g.set_layer_rows(l, rows, vals)
+        out = []
+        for part in (y0, y0[: max(1, len(y0) // 3)]):          # a second, smaller batch in the same buffers
+            g.set_input_dense(part, first)
+            res = g.infer()
+            out.append((g.categories().copy(), g.activations(), g.layer_live().copy(), res.survivors))
+        return out
+
+
+@pytest.mark.parametrize("env", [{}, {"SPDNN_RETIRE": "0"}, {"SPDNN_RESIDENT": "0"}, {"SPDNN_CHUNK_FIRST": "3"}, {"SPDNN_BITS_FIRST": "1"},
+                                 {"SPDNN_STAGE_TABLES": "0"}],
+                         ids=lambda e: ",".join(f"{k[6:]}={v}" for k, v in e.items()) or "default")
+@pytest.mark.parametrize("kind,n,b,L", [("random", 1024, 333, 26), ("random", 1024, 64, 9), ("random", 16384, 37, 18), ("radix16", 1024, 200, 61),
+                                        ("radix16", 4096, 97, 60), ("radix16", 16384, 65, 50), ("hole", 1024, 200, 24), ("general", 512, 150, 14),
+                                        ("all", 1024, 40, 12)])
+def test_retired_images_are_survivors(kind, n, b, L, env, monkeypatch, oracle):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    net = SyntheticNetwork(n, L, "radix16" if kind == "radix16" else "random")
+    bias, clip = float(net.bias), 32.0
+    layers = [(r, None) for r in rows_of(net)]
+    y0 = synthetic_images(n, b) if kind == "radix16" else mixed_density_images(n, b)
+    if kind == "hole":                       # one layer in mid-network does not keep the all-clip vector
+        rows = layers[13][0].copy()
+        rows[5] = -1
+        layers[13] = (rows, None)
+    if kind == "general":
+        rng = np.random.default_rng(7)
+        layers = [(r, rng.uniform(0.02, 0.2, r.shape).astype(np.float32)) for r, _ in layers]
+        bias = -0.25
+    if kind == "all":                        # every image at clip from the start, next to dead ones
+        y0[:] = clip
+        y0[::7] = 0.0
+    got = run(n, layers, bias, clip, y0, 11)
+    for part, (cats, act, live, survivors) in zip((y0, y0[: max(1, b // 3)]), got):
+        wc, wa, wl = oracle.infer(part, layers, bias, clip=clip, first_image=11)
+        assert np.array_equal(live, wl)
+        assert np.array_equal(cats, wc) and survivors == len(wc)
+        assert np.array_equal(act, wa)
