@@ -623,17 +623,7 @@ alt2_kernel(const ResArgs a) {
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    LayerArgs la;
-    la.yin = a.yin; la.yout = a.yout; la.tile_stride = a.tile_stride;
-    la.ctl_in = a.ctl_in; la.ctl_out = a.ctl_out; la.slot = a.slot; la.mask = a.mask;
-    la.ids0 = a.ids0; la.ids1 = a.ids1; la.counter = a.counter; la.work = a.work; la.status = a.status;
-    la.died_at = nullptr;
-    la.first_member_only = 0;
-    la.bias = a.bias; la.clip = a.clip;
-    la.xw = nullptr; la.nw = 0; la.gate = nullptr; la.gate_want = 0;
-    la.retire = a.retire;
-    la.retire.open = nullptr;
-    rebuild_worklist(la, live_in, ctl.ids_buf);
+    rebuild_worklist(chunk_layer_args(a), live_in, ctl.ids_buf);
 }
 
 }  // namespace spdnn_impl

@@ -405,6 +405,18 @@ int launch_generic(spdnn *c, const ResArgs &a, int grid, size_t smem, bool k32, 
                   : launch_resident_t<TI, 4, 0, false, false>(c, a, grid, smem);
 }
 
+template <int NT>
+int launch_inplace(spdnn *c, const ResArgs &a, int grid, size_t smem, bool k32, bool uniform) {
+    auto go = [&](auto kernel) -> int {
+        if (int rc = allow_max_dynamic_smem(c, kernel)) return rc;
+        kernel<<<grid, NT, smem, c->stream>>>(a);
+        CK(cudaGetLastError());
+        return SPDNN_OK;
+    };
+    if (k32) return uniform ? go(inplace_kernel<NT, 32, true>) : go(inplace_kernel<NT, 32, false>);
+    return uniform ? go(inplace_kernel<NT, 0, true>) : go(inplace_kernel<NT, 0, false>);
+}
+
 int launch_resident(spdnn *c, int ti, int ipt, const ResArgs &a, int grid, size_t smem, int mode, bool k32, bool uniform) {
     if (mode == kResAlt2) {
         // layers of at most 64 classes: blocks of 128 threads (one warp does the bit form; twice the blocks per SM)
@@ -423,6 +435,11 @@ int launch_resident(spdnn *c, int ti, int ipt, const ResArgs &a, int grid, size_
             case 8: return launch_alt2<8, 4, kThreads>(c, a, grid, smem, k32);
             default: return launch_alt2<4, 4, kThreads>(c, a, grid, smem, k32);
         }
+    }
+    if (ti == 32) {      // one thread per class of the widest layer (see inplace_kernel)
+        if (ipt <= 256) return launch_inplace<256>(c, a, grid, smem, k32, uniform);
+        if (ipt <= 512) return launch_inplace<512>(c, a, grid, smem, k32, uniform);
+        return launch_inplace<1024>(c, a, grid, smem, k32, uniform);
     }
     switch (ti) {
         case 16: return launch_generic<16>(c, a, grid, smem, k32, uniform);
@@ -503,6 +520,11 @@ inline int resident_rows(const DevRes &R) { return ((std::max(R.v_in, R.classes)
 // Dynamic shared memory of a resident block.  GENERIC chunks: two activation buffers and two
 // staged tables.  ALT2 chunks: two activation buffers, `tring` groups of 1 << gshift layer records
 // of `stride` bytes (the word buffers of the bit form live in the activation buffer that is free).
+// inplace_kernel: one activation buffer, eight threads per class and eight classes per thread of at most 1024 threads, two
+// buffers for the entries of four classes per warp.
+constexpr int kInplaceMaxClasses = 1024;
+inline int inplace_table_bytes(int k, bool uniform) { return 4 * (k + 4) * 4 * (uniform ? 1 : 2); }
+inline size_t inplace_smem_bytes(int rows, int warps, int table) { return (size_t)rows * 128 + (size_t)warps * 2 * table; }
 inline size_t resident_smem_bytes(int ti, int rows, int table) { return 2 * (size_t)rows * ti * 4 + 2 * (size_t)table; }
 inline size_t alt2_smem_bytes(int ti, int rows, int stride, int gshift, int tring) {
     return 2 * (size_t)rows * ti * 4 + (size_t)tring * ((size_t)stride << gshift);
@@ -513,7 +535,7 @@ inline size_t alt2_smem_bytes(int ti, int rows, int stride, int gshift, int trin
 // images still die, long once the survivors are stable), one launch per layer otherwise.
 struct Step {
     int first = 0, count = 1;      // layers [first, first + count)
-    int ti = 0, ipt = 4;           // resident chunk: images per block / per thread; ti == 0: per-layer kernel
+    int ti = 0, ipt = 4;           // resident chunk: images per block / per thread (GENERIC groups of 32: threads per block); ti == 0: per-layer kernel
     int rows = 0, table = 0;       // resident chunk: rows of one activation buffer, bytes per staged table
     // ALT2 chunk (alt2_kernel): packed table stream and its staging, word buffers of the bit form
     int stride = 0, gshift = 0, tring = 0, wring = 2, rows_w = 0, max_classes = 0;
@@ -560,16 +582,27 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
         if (c->res[l]) {
             const DevRes &R0 = *c->res[l];
             const bool k32 = (R0.k == 32);
+            int kmax = R0.k;               // most entries per class in the chunk
             auto fits = [&](int t_i, int r, int table) {
-                return resident_smem_bytes(t_i, r, table) + 2048 <= (size_t)c->smem_optin;
+                const size_t need = R0.mode == kResGeneric && t_i == 32 ? inplace_smem_bytes(r, 32, inplace_table_bytes(kmax, R0.uniform))
+                                                                       : resident_smem_bytes(t_i, r, table);
+                return need + 2048 <= (size_t)c->smem_optin;
             };
             int rows = resident_rows(R0), ti = 0, ipt = 4;
             // (images per block, images per thread) in order of preference; a form that would leave
             // most threads without a class (under half of what one pass of the block covers) is skipped
             static const int kAlt2[][2] = {{32, 8}, {16, 4}, {16, 8}, {8, 4}, {4, 4}};
-            static const int kGeneric[][2] = {{16, 4}, {8, 4}, {4, 4}};
+            static const int kGeneric[][2] = {{32, 4}, {16, 4}, {8, 4}, {4, 4}};
             const int (*cand)[2] = R0.mode == kResAlt2 ? kAlt2 : kGeneric;
-            const int ncand = R0.mode == kResAlt2 ? 5 : 3;
+            const int ncand = R0.mode == kResAlt2 ? 5 : 4;
+            // GENERIC groups: as many images as still give every SM a block; a block's time grows with its images, so a
+            // small batch is faster in smaller groups on more SMs ...
+            int most = 32;
+            if (R0.mode == kResGeneric) {
+                while (most > 4 && c->tiles_cap * (32 / most) < c->sm_count) most /= 2;
+                // ... and so are the few images that are left when most have been retired
+                if (c->retire && l >= c->settle_from + c->chunk_first && generic_chunks > 2) most = std::max(4, most >> (generic_chunks - 2));
+            }
             // First launch of a pass that reads the input in place.  A layer that reads all N rows to compute
             // few classes is mostly loading: it pays only with several blocks of at least 8 images per SM, so
             // that one block's loads overlap another's arithmetic -- it takes the largest group that leaves
@@ -581,7 +614,8 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
             for (int pass = (dense_wanted && wide_few) ? 0 : 1; pass < 2 && !ti; ++pass)
                 for (int q = 0; q < ncand; ++q) {
                     const int t_i = cand[q][0], i_pt = cand[q][1];
-                    if (t_i > c->res_ti_max || i_pt > c->res_ipt_max || !fits(t_i, rows, 0)) continue;
+                    if (t_i > c->res_ti_max || i_pt > c->res_ipt_max || t_i > most || !fits(t_i, rows, 0)) continue;
+                    if (R0.mode == kResGeneric && t_i == 32 && R0.classes > kInplaceMaxClasses) continue;
                     if (i_pt == 8 && R0.classes * 2 < kThreads * i_pt / t_i) continue;
                     if (pass == 0 && (t_i < 8 || resident_smem_bytes(t_i, rows, 0) * 3 > (size_t)c->smem_optin)) continue;
                     ti = t_i; ipt = i_pt;
@@ -595,14 +629,17 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                     const DevRes &M = *c->res[l + f];
                     if (M.mode != R0.mode || M.uniform != R0.uniform || (M.k == 32) != k32) break;
                     const int r2 = std::max(rows, resident_rows(M));
-                    if (!fits(ti, r2, 0)) break;
+                    const int k_before = kmax;
+                    kmax = std::max(kmax, M.k);
+                    if (!fits(ti, r2, 0) || (R0.mode == kResGeneric && ti == 32 && M.classes > kInplaceMaxClasses)) { kmax = k_before; break; }
                     rows = r2;
                     blob = std::max(blob, M.blob_bytes);
                     maxc = std::max(maxc, M.classes);
                     ++f;
                 }
                 int tb = (blob + 127) / 128 * 128;
-                if (!(c->stage_tables && fits(ti, rows, tb))) tb = 0;
+                if (R0.mode == kResGeneric && ti == 32) tb = inplace_table_bytes(kmax, R0.uniform);
+                else if (!(c->stage_tables && fits(ti, rows, tb))) tb = 0;
                 if (R0.mode == kResAlt2) {
                     // packed stream: groups of up to 32 layers per bulk copy (what a group costs besides its
                     // layers -- waiting for the copy, checking the result -- is spread over them), the next group
@@ -666,6 +703,7 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                     }
                 }
                 if (R0.mode == kResGeneric) {
+                    if (ti == 32) ipt = maxc <= 256 ? 256 : maxc <= 512 ? 512 : 1024;      // inplace_kernel: threads per block
                     // count_kernel pre-pass for tiles that are saturated already: uniform weight, 32 entries per class
                     // (its adder tree is built for 32), the two word buffers in shared memory
                     bool k32_all = k32 && R0.uniform;
@@ -744,7 +782,8 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
 // (0: binary, read the words; 1: read the float tiles), and each checks the flag at entry:
 //   kFrontWords   layer 0 runs in the per-layer kernel, whose BITS variant gathers from the words;
 //   kFrontExpand  the pass starts with a resident chunk: the words are expanded to float tiles first.
-enum { kFrontNone = 0, kFrontWords = 1, kFrontExpand = 3 };
+//   kFrontInPlace the pass starts with a GENERIC resident chunk, which reads words or floats by the flag itself.
+enum { kFrontNone = 0, kFrontWords = 1, kFrontInPlace = 2, kFrontExpand = 3 };
 
 int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
     c->last_group = 0;
@@ -756,7 +795,10 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
         if (plan[0].ti == 0) {
             front = kFrontWords;
         } else {
-            front = kFrontExpand;
+            // a GENERIC chunk reads the words itself; an ALT2 chunk and a pre-pass want them as float tiles
+            front = c->res[0]->mode == kResGeneric && plan[0].bits_threads == 0 ? kFrontInPlace : kFrontExpand;
+        }
+        if (front == kFrontExpand) {
             const long long warps = (long long)c->tiles_cap * c->n;
             const int grid = (int)std::min<long long>((warps + 7) / 8, (long long)c->sm_count * 32);
             words_to_tiles_kernel<<<std::max(1, grid), 256, 0, c->stream>>>(c->xw, c->nw, c->n, c->tiles_cap, c->y[0], c->tile_stride,
@@ -805,12 +847,14 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
             const int grid = std::max(1, (c->tiles_cap * 32 + st.ti - 1) / st.ti);
             const bool alt2 = (R0.mode == kResAlt2);
             const size_t smem = alt2 ? alt2_smem_bytes(st.ti, st.rows, st.stride, st.gshift, st.tring)
-                                     : resident_smem_bytes(st.ti, st.rows, st.table);
+                              : st.ti == 32 ? inplace_smem_bytes(st.rows, st.ipt / 32, st.table) : resident_smem_bytes(st.ti, st.rows, st.table);
             a.bit_ok = (alt2 && c->bit_form && c->clip > 0.0f && st.wring >= 2) ? 1 : 0;
             a.tile_done = nullptr; a.wwords = 0;
             a.cache = nullptr; a.rec_of = nullptr; a.cache_records = 0;
             a.period = st.period; a.period_from = st.period_from;
             a.gate = nullptr; a.gate_want = 0;
+            a.xw = step == 0 && front == kFrontInPlace ? c->xw : nullptr;
+            a.xw_flag = c->in_flag; a.nw = c->nw;
             a.retire = retire;
             a.settle_from = c->retire ? std::max(0, c->settle_from - l) : st.count + 1;
             if (alt2 && st.bits_threads > 0) {

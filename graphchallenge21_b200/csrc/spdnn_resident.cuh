@@ -104,6 +104,11 @@ struct ResArgs {
     // The chunk's tables repeat: layer q + period uses the tables of layer q for every q >= period_from (0: no period).
     // Saturated activations that one period maps onto themselves are then a fixed point of all later periods.
     int period, period_from;
+    // First chunk of a pass, GENERIC tables: where *xw_flag is 0 the input is binary and is read from its words (bit i of
+    // xw[tile * nw + r] = image i of the tile has neuron r set) instead of the float tiles; nullptr: float tiles
+    const uint32_t *xw;
+    const int32_t *xw_flag;
+    int nw;
     // the launch runs only when *gate == gate_want (nullptr: always), see LayerArgs
     const int32_t *gate;
     int gate_want;
@@ -289,6 +294,21 @@ __device__ __forceinline__ float finish_output(float sum, float bias, float clip
     return fminf(fmaxf(__fadd_rn(sum, bias), 0.0f), clip);
 }
 
+// What the work-list rebuild at the end of a chunk needs, as the per-layer kernel's arguments.
+__device__ __forceinline__ LayerArgs chunk_layer_args(const ResArgs &a) {
+    LayerArgs la;
+    la.yin = a.yin; la.yout = a.yout; la.tile_stride = a.tile_stride;
+    la.ctl_in = a.ctl_in; la.ctl_out = a.ctl_out; la.slot = a.slot; la.mask = a.mask;
+    la.ids0 = a.ids0; la.ids1 = a.ids1; la.counter = a.counter; la.work = a.work; la.status = a.status;
+    la.died_at = nullptr;
+    la.first_member_only = 0;
+    la.bias = a.bias; la.clip = a.clip;
+    la.xw = nullptr; la.nw = 0; la.gate = nullptr; la.gate_want = 0;
+    la.retire = a.retire;
+    la.retire.open = nullptr;
+    return la;
+}
+
 // Load phase of a first launch that reads the caller's row-major input in place, for layers whose
 // value ids are the neurons themselves: image j0 + i, rows [0, rows) -> cur[phys_row(r)][i].
 // A warp covers 32 / TI groups of four consecutive rows for each of the TI images with one 16-byte
@@ -406,6 +426,7 @@ resident_kernel(const ResArgs a) {
             const ResLayer L0 = a.layers[0];
             if (!ctl.identity && rgrp == 0 && valid) move_id(ctl, a.ids0, a.ids1, j, src);
             const float *const pimg = dense ? dense + (size_t)src * a.n : a.yin + (size_t)(src >> 5) * a.tile_stride + (src & 31);
+            const uint32_t *const words = a.xw != nullptr && *a.xw_flag == 0 ? a.xw + (size_t)(src >> 5) * a.nw : nullptr;
             const bool fast_dense = dense && !L0.rep && L0.v_in == a.n && (a.n & 3) == 0 && (reinterpret_cast<size_t>(dense) & 15) == 0;
             if (fast_dense) load_dense_rows<TI, NT, false, true>(dense, a.n, j0, live_in, L0.v_in, cur, a.clip);
             for (int v0 = rgrp; v0 < L0.v_in && !fast_dense; v0 += RPP * UNR) {
@@ -419,7 +440,8 @@ resident_kernel(const ResArgs a) {
                     if (dense) e[t] >>= 5;
                 }
 #pragma unroll
-                for (int t = 0; t < UNR; ++t) x[t] = valid ? __ldg(pimg + e[t]) : 0.0f;
+                for (int t = 0; t < UNR; ++t)
+                    x[t] = !valid ? 0.0f : words ? (float)((__ldg(words + (e[t] >> 5)) >> (src & 31)) & 1u) : __ldg(pimg + e[t]);
 #pragma unroll
                 for (int t = 0; t < UNR; ++t) {
                     const int v = v0 + t * RPP;
@@ -622,17 +644,220 @@ resident_kernel(const ResArgs a) {
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    LayerArgs la;
-    la.yin = a.yin; la.yout = a.yout; la.tile_stride = a.tile_stride;
-    la.ctl_in = a.ctl_in; la.ctl_out = a.ctl_out; la.slot = a.slot; la.mask = a.mask;
-    la.ids0 = a.ids0; la.ids1 = a.ids1; la.counter = a.counter; la.work = a.work; la.status = a.status;
-    la.died_at = nullptr;
-    la.first_member_only = 0;
-    la.bias = a.bias; la.clip = a.clip;
-    la.xw = nullptr; la.nw = 0; la.gate = nullptr; la.gate_want = 0;
-    la.retire = a.retire;
-    la.retire.open = nullptr;
-    rebuild_worklist(la, live_in, ctl.ids_buf);
+    rebuild_worklist(chunk_layer_args(a), live_in, ctl.ids_buf);
+}
+
+// ---- inplace_kernel: GENERIC chunks in groups of 32 images ------------------------------------------------------
+//
+// What bounds a GENERIC layer is reading K rows per class out of shared memory.  With 32 images a row is the 128 bytes
+// that the banks span, so the eight lanes of a class read all banks once and no two rows of a warp's load get in each
+// other's way (with 16 images the two rows that share a wavefront hit the same half of the banks half of the time).  Two
+// buffers of 32 images do not fit at 1024 neurons; ONE does, with the outputs of a layer kept in registers (32 floats a
+// thread, eight classes) until every thread has read its inputs: two barriers per layer instead of one.
+// Tables: a warp takes four classes at a time and fetches the entries of its next four (a few hundred bytes, of the
+// next layer's first ones behind the last) into a buffer of its own while it adds, so that no load of the loop waits for L2
+// (read in place, that wait was a tenth of the kernel).
+// 60000 images, 1024 neurons, 32 random rows per column, layers 0..7: 3812 us with two buffers of 16 images, 2948 with one of
+// 32, 2678 with the entries fetched ahead; eight times 217 us is what reading the rows takes at 128 bytes a clock.
+constexpr int kInplaceClassesPerThread = 8;
+
+// Threads: one per class of the chunk's widest layer (256, 512 or 1024), so that eight classes per thread and eight
+// lanes per class cover a layer.  Dynamic shared memory: buf_rows * 128 bytes, then two buffers of table_bytes per warp.
+template <int NT, int KT, bool UNIFORM>
+__global__ void __launch_bounds__(NT, 1024 / NT) inplace_kernel(const ResArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ unsigned int s_alive[3];
+    __shared__ unsigned int s_open[3];           // images with an output of layer li % 3 that is not clip
+    __shared__ int s_last;
+    constexpr int RS = 128, CPP = NT / 8;        // bytes per row; classes per pass of the block
+    if (a.gate != nullptr && *a.gate != a.gate_want) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sub = tid & 7, grp = tid >> 3;
+    const LoopCtl ctl = *a.ctl_in;
+    const int live_in = ctl.live, tile = blockIdx.x;
+    const bool tile_finished = a.tile_done != nullptr && tile * 32 < live_in && a.tile_done[tile] != 0;
+    if (tile * 32 < live_in && !tile_finished) {
+        const bool valid = tile * 32 + lane < live_in;
+        {
+            // one row per value id: a lane owns an image, a warp a row; up to UNR loads in flight
+            constexpr int UNR = 8;
+            const float *const dense = a.dense_in ? *a.dense_in : nullptr;
+            const uint32_t *const words = a.xw != nullptr && *a.xw_flag == 0 ? a.xw + (size_t)tile * a.nw : nullptr;
+            const int j = valid ? tile * 32 + lane : tile * 32;
+            const int src = ctl.identity ? j : __ldg(a.slot + j);
+            if (!ctl.identity && warp == 0 && valid) move_id(ctl, a.ids0, a.ids1, j, src);
+            const float *const pimg = dense ? dense + (size_t)src * a.n : a.yin + (size_t)(src >> 5) * a.tile_stride + (src & 31);
+            const ResLayer L0 = a.layers[0];
+            for (int v0 = warp; v0 < L0.v_in; v0 += (NT / 32) * UNR) {
+                int e[UNR];
+                float x[UNR];
+#pragma unroll
+                for (int t = 0; t < UNR; ++t) {
+                    const int v = min(v0 + t * (NT / 32), L0.v_in - 1);
+                    // element of row r: r * 32 floats into a tile's column, r floats into a row-major image
+                    e[t] = L0.rep ? __ldg(L0.rep + v) : v * 32;
+                    if (dense) e[t] >>= 5;
+                }
+#pragma unroll
+                for (int t = 0; t < UNR; ++t)
+                    x[t] = !valid ? 0.0f : words ? (float)((__ldg(words + (e[t] >> 5)) >> lane) & 1u) : __ldg(pimg + e[t]);
+#pragma unroll
+                for (int t = 0; t < UNR; ++t) {
+                    const int v = v0 + t * (NT / 32);
+                    if (v < L0.v_in) *reinterpret_cast<float *>(smem + resident_phys_row(v) * RS + lane * 4) = x[t];
+                }
+            }
+            // rows v_in .. even(v_in) + 1 are the zero rows padded table entries point at
+            const int ve = (L0.v_in + 1) & ~1;
+            for (int r = L0.v_in + warp; r < ve + 2; r += NT / 32)
+                *reinterpret_cast<float *>(smem + (r < ve ? resident_phys_row(r) : r) * RS + lane * 4) = 0.0f;
+            if (tid == 0) s_alive[0] = s_open[0] = 0u;
+        }
+        unsigned int alive = __ballot_sync(0xffffffffu, valid), open_now = 0xffffffffu;
+        const bool force_dead = a.bias > 0.0f;
+        const unsigned char *const in = smem + sub * 16;
+        unsigned char *const wtab = smem + (size_t)a.buf_rows * RS + (size_t)warp * 2 * a.table_bytes;
+        // the entries of the warp's four classes of a pass, into its buffer `buf`: row numbers, then weights
+        auto fetch = [&](const int32_t *T, int classes, int kp, int p, int buf) {
+            const int u0 = p * CPP + warp * 4, pieces = max(0, min(4, classes - u0)) * (kp / 4);      // of 16 bytes
+            const int4 *const from = reinterpret_cast<const int4 *>(T + 4 + (size_t)u0 * kp);
+            unsigned char *const to = wtab + buf * a.table_bytes;
+            for (int q = lane; q < pieces; q += 32) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to + q * 16)), "l"(from + q) : "memory");
+                if (!UNIFORM)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to + a.table_bytes / 2 + q * 16)),
+                                 "l"(from + (size_t)classes * (kp / 4) + q)
+                                 : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        int li = 0, last_classes = 0, tbuf = 0;
+        bool settled = false;
+        const int32_t *T = a.layers[0].blob;
+        int classes = a.layers[0].classes, k = a.layers[0].k;
+        float w = a.layers[0].w;
+        fetch(T, classes, k + 4, 0, 0);
+        __syncthreads();
+        while (li < a.nlayers) {
+            const int kp = k + 4;
+            // the next layer's tables
+            const ResLayer LN = a.layers[min(li + 1, a.nlayers - 1)];
+            const unsigned int al = alive >> (4 * sub);
+            unsigned int bits = 0u, open = 0u;
+            float4 out[kInplaceClassesPerThread];
+#pragma unroll
+            for (int p = 0; p < kInplaceClassesPerThread; ++p) {
+                const int u = p * CPP + grp;
+                out[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (p * CPP < classes) {         // (for the whole block)
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
+                    __syncwarp();
+                    tbuf ^= 1;                   // this pass reads buffer tbuf ^ 1
+                    if (p + 1 < kInplaceClassesPerThread && (p + 1) * CPP < classes) fetch(T, classes, kp, p + 1, tbuf);
+                    else if (li + 1 < a.nlayers) fetch(LN.blob, LN.classes, LN.k + 4, 0, tbuf);
+                }
+                if (u < classes) {
+                    const int4 *const rows = reinterpret_cast<const int4 *>(wtab + (tbuf ^ 1) * a.table_bytes) + (lane >> 3) * (kp / 4);
+                    const float4 *const vals = reinterpret_cast<const float4 *>(wtab + (tbuf ^ 1) * a.table_bytes + a.table_bytes / 2) + (lane >> 3) * (kp / 4);
+                    Acc4 acc = acc_zero();
+#pragma unroll 2
+                    for (int i = 0; i < (KT > 0 ? KT : k) / 4; ++i) {
+                        const int4 r = rows[i];
+                        float4 x0 = *reinterpret_cast<const float4 *>(in + r.x * RS), x1 = *reinterpret_cast<const float4 *>(in + r.y * RS);
+                        float4 x2 = *reinterpret_cast<const float4 *>(in + r.z * RS), x3 = *reinterpret_cast<const float4 *>(in + r.w * RS);
+                        if (!UNIFORM) {
+                            const float4 q = vals[i];
+                            x0 = mul4(x0, q.x); x1 = mul4(x1, q.y); x2 = mul4(x2, q.z); x3 = mul4(x3, q.w);
+                        }
+                        acc_add(acc, acc_from(x0)); acc_add(acc, acc_from(x1)); acc_add(acc, acc_from(x2)); acc_add(acc, acc_from(x3));
+                    }
+                    float4 y = acc_get(acc);
+                    if (UNIFORM) y = mul4(y, w);
+                    y = make_float4(finish_output(y.x, a.bias, a.clip), finish_output(y.y, a.bias, a.clip), finish_output(y.z, a.bias, a.clip),
+                                    finish_output(y.w, a.bias, a.clip));
+                    // dead images stay dead: with bias <= 0 an all-zero image stays all-zero by itself
+                    if (force_dead) {
+                        if (!(al & 1u)) y.x = 0.0f;
+                        if (!(al & 2u)) y.y = 0.0f;
+                        if (!(al & 4u)) y.z = 0.0f;
+                        if (!(al & 8u)) y.w = 0.0f;
+                    }
+                    bits |= (y.x != 0.0f ? 1u : 0u) | (y.y != 0.0f ? 2u : 0u) | (y.z != 0.0f ? 4u : 0u) | (y.w != 0.0f ? 8u : 0u);
+                    open |= (y.x != a.clip ? 1u : 0u) | (y.y != a.clip ? 2u : 0u) | (y.z != a.clip ? 4u : 0u) | (y.w != a.clip ? 8u : 0u);
+                    out[p] = y;
+                }
+            }
+            const unsigned int wm = __reduce_or_sync(0xffffffffu, bits << (4 * sub)), om = __reduce_or_sync(0xffffffffu, open << (4 * sub));
+            if (lane == 0 && wm) atomicOr(&s_alive[li % 3], wm);
+            if (lane == 0 && om) atomicOr(&s_open[li % 3], om);
+            if (tid == 0) s_alive[(li + 1) % 3] = s_open[(li + 1) % 3] = 0u;      // last read after layer li - 2
+            __syncthreads();                     // every thread has read its inputs
+#pragma unroll
+            for (int p = 0; p < kInplaceClassesPerThread; ++p) {
+                const int u = p * CPP + grp;
+                if (u < classes) *reinterpret_cast<float4 *>(smem + resident_phys_row(u) * RS + sub * 16) = out[p];
+            }
+            const int ue = (classes + 1) & ~1;   // the next layer's zero rows
+            for (int r = classes + grp; r < ue + 2; r += CPP)
+                *reinterpret_cast<float4 *>(smem + (r < ue ? resident_phys_row(r) : r) * RS + sub * 16) = make_float4(0, 0, 0, 0);
+            const unsigned int now = s_alive[li % 3] & alive;
+            open_now = s_open[li % 3];
+            if (tid == 0 && now != alive) atomicAdd(a.died_at + li, __popc(alive & ~now));
+            alive = now;
+            last_classes = classes;
+            T = LN.blob; classes = LN.classes; k = LN.k; w = LN.w;
+            ++li;
+            __syncthreads();
+            if (alive == 0u) break;
+            // every image still alive has reached its result: the rest of the chunk changes nothing
+            if ((alive & open_now) == 0u && li >= a.settle_from && li < a.nlayers) { settled = true; break; }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // images that have reached their result leave the work list; what is left of the tile's images is stored
+        const unsigned int retired = a.retire.on ? alive & ~open_now : 0u;
+        alive &= ~retired;
+        if (warp == 0 && retired != 0u) {
+            retire_images(a.retire, ctl.ids_buf ? a.ids1 : a.ids0, tile * 32, retired);
+            if (tid == 0) atomicAdd(a.retire.count, (unsigned int)__popc(retired));
+        }
+        if (alive != 0u) {
+            if (settled) li = a.nlayers;
+            const ResLayer LL = a.layers[li - 1];
+            if (settled) last_classes = LL.classes;
+            float *const out = a.yout + (size_t)tile * a.tile_stride + lane;
+            const float top = (alive >> lane) & 1u ? a.clip : 0.0f;
+            // one row per class, or all member rows; the offsets of SU classes are looked up together
+            constexpr int SU = 8;
+            for (int u0 = warp; u0 < last_classes; u0 += (NT / 32) * SU) {
+                int mb[SU], me[SU];
+#pragma unroll
+                for (int t = 0; t < SU; ++t) {
+                    const int u = min(u0 + t * (NT / 32), last_classes - 1);
+                    mb[t] = LL.mem_ptr ? __ldg(LL.mem_ptr + u) : u;
+                    me[t] = LL.mem_ptr && !a.reps_only ? __ldg(LL.mem_ptr + u + 1) : mb[t] + 1;
+                }
+#pragma unroll
+                for (int t = 0; t < SU; ++t) {
+                    const int u = u0 + t * (NT / 32);
+                    if (u >= last_classes) break;
+                    const float y = settled ? top : *reinterpret_cast<const float *>(smem + resident_phys_row(u) * RS + lane * 4);
+                    for (int m = mb[t]; m < me[t]; ++m) out[LL.mem_ptr ? __ldg(LL.mem + m) : m * 32] = y;
+                }
+            }
+            if (tid == 0) atomicOr(a.mask + tile, alive);
+        }
+    }
+
+    // ---- last block done: rebuild the work list
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        s_last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    rebuild_worklist(chunk_layer_args(a), live_in, ctl.ids_buf);
 }
 
 }  // namespace spdnn_impl

@@ -1,0 +1,63 @@
+"""GPU tests of the group sizes of GENERIC chunks: the batch decides how many images a block holds (32 with one buffer and
+the outputs in registers, 16, 8 or 4 with two), every size against the oracle, bit for bit."""
+import numpy as np
+import pytest
+
+from conftest import mixed_density_images
+from graphchallenge21_b200 import SpDNN
+from graphchallenge21_b200.generator import SyntheticNetwork
+from graphchallenge21_b200.network import pack_bits
+
+pytestmark = pytest.mark.gpu
+
+
+def network(n, L, k, seed):
+    """Ragged columns (every tenth entry missing), every weight another value."""
+    rng = np.random.default_rng(seed)
+    out = []
+    for _ in range(L):
+        rows = np.sort(np.argpartition(rng.random((n, n)), k, axis=1)[:, :k], axis=1).astype(np.int32)
+        rows[rng.random(rows.shape) < 0.1] = -1
+        out.append((rows, rng.uniform(0.02, 0.2, rows.shape).astype(np.float32)))
+    return out
+
+
+@pytest.mark.parametrize("batch", [4737, 2400, 1190, 70])           # 32, 16, 8 and 4 images a block on 148 SMs
+@pytest.mark.parametrize("n,k,L", [(96, 20, 11), (256, 37, 9), (512, 32, 9), (700, 9, 4), (1024, 32, 10)])
+def test_general_weights(n, k, L, batch, oracle):
+    layers = network(n, L, k, n + k)
+    y0 = mixed_density_images(n, batch)
+    y0[::5] *= np.float32(0.7)
+    want_c, want_a, want_l = oracle.infer(y0, layers, -0.25, first_image=2)
+    with SpDNN(n, L, -0.25) as g:
+        for l, (rows, vals) in enumerate(layers):
+            g.set_layer_rows(l, rows, vals)
+        g.set_input_dense(y0, 2)
+        res = g.infer()
+        assert np.array_equal(g.layer_live(), want_l) and res.survivors == len(want_c)
+        assert np.array_equal(g.categories(), want_c)
+        assert np.array_equal(g.activations(), want_a)
+
+
+@pytest.mark.parametrize("how", ["dense", "bits", "grey"])
+@pytest.mark.parametrize("bias", [-0.3, 0.05])
+@pytest.mark.parametrize("batch", [4737, 2400, 300])
+def test_binary_words_are_read_in_place(batch, bias, how, oracle):
+    n, L = 1024, 9
+    net = SyntheticNetwork(n, L, "random", bias=bias)
+    layers = [(net.layer_rows(l), None) for l in range(L)]
+    y0 = mixed_density_images(n, batch)
+    if how == "grey":
+        y0[-1] *= np.float32(0.5)                    # one image that is not binary: all take the float tiles
+    want_c, want_a, want_l = oracle.infer(y0, layers, bias)
+    with SpDNN(n, L, bias) as g:
+        g.set_network(net)
+        for _ in range(2):
+            if how == "bits":
+                g.set_input_bits(pack_bits(y0))
+            else:
+                g.set_input_dense(y0)
+            g.infer()
+            assert np.array_equal(g.layer_live(), want_l)
+            assert np.array_equal(g.categories(), want_c)
+            assert np.array_equal(g.activations(), want_a)
