@@ -125,7 +125,8 @@ struct spdnn {
     int chunk_growth_generic = 2;      // GENERIC chunks grow more slowly: a tile that is not saturated when its chunk starts
                                        // stays in the float form to the chunk's end, and that form costs 32 gathers per output
     int nsteps = 0;                    // launches of the last captured schedule
-    std::vector<int32_t> host_died, host_live;
+    std::vector<int32_t> host_live;
+    HostReport report{};               // page-locked host memory the last launch of a pass writes its results to (ids: sized with the batch)
     int32_t *slot = nullptr;
     uint32_t *mask = nullptr;
     unsigned char *tile_done = nullptr;   // [tiles] verdict of the bits_kernel pre-pass of an ALT2 chunk
@@ -185,7 +186,6 @@ struct spdnn {
     int input_kind = 0;
     int cpi_override = 0, grid_override = 0;
 
-    std::vector<LoopCtl> host_ctl;
     spdnn_stats_t stats{};
     int64_t prep_launches = 0;
     std::string err;
@@ -211,13 +211,18 @@ int fail(spdnn *c, int code, const char *fmt, ...) {
                         __FILE__, __LINE__);                                                          \
     } while (0)
 
+// has_floats lies behind in_flag in one allocation, so that one memset resets both
+constexpr size_t kMarksOffset = 16;
+
 int free_buffers(spdnn *c) {
     cudaFree(c->y[0]); cudaFree(c->y[1]); cudaFree(c->slot); cudaFree(c->mask); cudaFree(c->tile_done);
-    cudaFree(c->ids[0]); cudaFree(c->ids[1]); cudaFree(c->xw); cudaFree(c->has_floats);
+    cudaFree(c->ids[0]); cudaFree(c->ids[1]); cudaFree(c->xw); cudaFree(c->in_flag);
     cudaFree(c->open_mask); cudaFree(c->settled); cudaFree(c->working); cudaFree(c->work_of);
     c->open_mask = c->settled = c->working = nullptr; c->work_of = nullptr;
     c->y[0] = c->y[1] = nullptr; c->slot = nullptr; c->mask = nullptr; c->ids[0] = c->ids[1] = nullptr;
-    c->tile_done = nullptr; c->xw = nullptr; c->has_floats = nullptr;
+    c->tile_done = nullptr; c->xw = nullptr; c->has_floats = nullptr; c->in_flag = nullptr;
+    cudaFreeHost(c->report.ids);
+    c->report.ids = nullptr;
     c->tiles_cap = 0;
     return SPDNN_OK;
 }
@@ -225,6 +230,7 @@ int free_buffers(spdnn *c) {
 int ensure_capacity(spdnn *c, int batch) {
     const int tiles = (batch + 31) / 32;
     if (tiles <= c->tiles_cap) return SPDNN_OK;
+    CK(cudaStreamSynchronize(c->stream));      // (the last launch of a pass in flight writes to host memory that goes)
     free_buffers(c);
     c->graph_dirty = true;
     const size_t ybytes = (size_t)tiles * (size_t)c->tile_stride * sizeof(float);
@@ -233,6 +239,7 @@ int ensure_capacity(spdnn *c, int batch) {
         CK(cudaMemsetAsync(c->y[i], 0, ybytes, c->stream));      // incl. the permanent zero row of every tile
         CK(cudaMalloc(&c->ids[i], sizeof(int32_t) * (size_t)tiles * 32));
     }
+    CK(cudaMallocHost(&c->report.ids, sizeof(int32_t) * (size_t)tiles * 32));
     CK(cudaMalloc(&c->slot, sizeof(int32_t) * (size_t)tiles * 32));
     CK(cudaMalloc(&c->mask, sizeof(uint32_t) * (size_t)tiles));
     CK(cudaMemsetAsync(c->mask, 0, sizeof(uint32_t) * (size_t)tiles, c->stream));
@@ -245,8 +252,9 @@ int ensure_capacity(spdnn *c, int batch) {
     CK(cudaMemsetAsync(c->tile_done, 0, (size_t)tiles, c->stream));
     CK(cudaMalloc(&c->xw, sizeof(uint32_t) * (size_t)tiles * c->nw));
     CK(cudaMemsetAsync(c->xw, 0, sizeof(uint32_t) * (size_t)tiles * c->nw, c->stream));     // incl. the zero words behind the neurons
-    CK(cudaMalloc(&c->has_floats, (size_t)tiles));
-    CK(cudaMemsetAsync(c->has_floats, 0, (size_t)tiles, c->stream));
+    CK(cudaMalloc(&c->in_flag, kMarksOffset + (size_t)tiles));
+    CK(cudaMemsetAsync(c->in_flag, 0, kMarksOffset + (size_t)tiles, c->stream));
+    c->has_floats = reinterpret_cast<unsigned char *>(c->in_flag) + kMarksOffset;
     c->tiles_cap = tiles;
     return SPDNN_OK;
 }
@@ -280,8 +288,9 @@ int begin_input(spdnn *c, int batch, int first_global_id) {
     CK(cudaEventRecord(c->ev_prep0, c->stream));
     // the input counts as binary until a conversion kernel sees another value; with the binary front
     // switched off every input takes the float path
-    CK(cudaMemsetAsync(c->in_flag, c->binary_front ? 0 : 1, 1, c->stream));
-    CK(cudaMemsetAsync(c->has_floats, 0, (size_t)((batch + 31) / 32 > 0 ? (batch + 31) / 32 : 1), c->stream));
+    const size_t marks = (size_t)((batch + 31) / 32 > 0 ? (batch + 31) / 32 : 1);
+    CK(cudaMemsetAsync(c->in_flag, 0, kMarksOffset + marks, c->stream));
+    if (!c->binary_front) CK(cudaMemsetAsync(c->in_flag, 1, 1, c->stream));
     return SPDNN_OK;
 }
 
@@ -998,12 +1007,13 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
         }
     }
     c->nsteps = (int)plan.size();
-    finalize_ids_kernel<<<std::max(1, std::min(c->tiles_cap, 4 * c->sm_count)), 256, 0, c->stream>>>(c->ctl + c->nsteps, c->slot,
-                                                                                             c->ids[0], c->ids[1], c->working, c->first_cell);
+    finalize_kernel<<<std::max(1, std::min(c->tiles_cap, 4 * c->sm_count)), 256, 0, c->stream>>>(
+        c->ctl, c->nsteps, c->slot, c->ids[0], c->ids[1], c->died_at, c->layers, c->status, c->report, c->working,
+        c->first_cell);
     CK(cudaGetLastError());
     if (c->retires) {
-        merge_settled_kernel<<<(c->tiles_cap + kMergeWords - 1) / kMergeWords, 256, 0, c->stream>>>(c->ctl + c->nsteps, c->ids[0], c->ids[1], c->working, c->settled, c->tiles_cap,
-                                                        c->first_cell, c->work_of);
+        merge_settled_kernel<<<(c->tiles_cap + kMergeWords - 1) / kMergeWords, 256, 0, c->stream>>>(c->ctl + c->nsteps, c->working, c->settled, c->tiles_cap,
+                                                        c->first_cell, c->report.ids, c->work_of);
         CK(cudaGetLastError());
         c->extra_launches += 1;
     }
@@ -1167,13 +1177,19 @@ int spdnn_create(spdnn_t **out, int device, int neurons, int layers, float bias,
     CK(cudaMalloc(&c->dense_cell, sizeof(const float *)));
     CK(cudaMemset(c->dense_cell, 0, sizeof(const float *)));
     CK(cudaMemset(c->status, 0, sizeof(int32_t)));
-    CK(cudaMalloc(&c->in_flag, sizeof(int32_t)));
-    CK(cudaMemset(c->in_flag, 0, sizeof(int32_t)));
     CK(cudaMalloc(&c->died_at, sizeof(int32_t) * (size_t)layers));
     CK(cudaMemset(c->died_at, 0, sizeof(int32_t) * (size_t)layers));
     CK(cudaMalloc(&c->res_table, sizeof(ResLayer) * (size_t)layers));
-    c->host_ctl.resize(layers + 1);
-    c->host_died.assign(layers, 0);
+    {
+        // one block: the records per launch boundary, the deaths per layer, the status
+        unsigned char *block = nullptr;
+        const size_t ctl_bytes = sizeof(LoopCtl) * (size_t)(layers + 1);
+        CK(cudaMallocHost(&block, ctl_bytes + sizeof(int32_t) * ((size_t)layers + 1)));
+        memset(block, 0, ctl_bytes + sizeof(int32_t) * ((size_t)layers + 1));
+        c->report.ctl = reinterpret_cast<LoopCtl *>(block);
+        c->report.died_at = reinterpret_cast<int32_t *>(block + ctl_bytes);
+        c->report.status = c->report.died_at + layers;
+    }
     c->host_live.assign(layers, 0);
     {
         int optin = 0;
@@ -1237,8 +1253,9 @@ void spdnn_destroy(spdnn_t *c) {
     for (int kind = 0; kind < 2; ++kind)
         if (c->graph_exec[kind]) cudaGraphExecDestroy(c->graph_exec[kind]);
     cudaFree(c->dense_cell); cudaFree(c->first_cell);
+    cudaFreeHost(c->report.ctl);
     free_buffers(c);
-    cudaFree(c->ctl); cudaFree(c->counter); cudaFree(c->status); cudaFree(c->stage); cudaFree(c->in_flag);
+    cudaFree(c->ctl); cudaFree(c->counter); cudaFree(c->status); cudaFree(c->stage);
     cudaFree(c->died_at); cudaFree(c->res_table);
     for (unsigned char *p : c->streams) cudaFree(p);
     c->layer.clear();
@@ -1409,9 +1426,8 @@ int spdnn_set_input_dense_device(spdnn_t *c, const float *y0_dev, int batch, int
         c->input_kind = 1;
         return end_input(c);
     }
+    // (converted in one piece: the flag is final when the float form of the tiles is written, none is left to repair)
     rc = convert_dense_device(c, y0_dev, batch, 0);
-    if (rc) return rc;
-    rc = repair_float_tiles(c);
     if (rc) return rc;
     return end_input(c);
 }
@@ -1445,8 +1461,10 @@ int spdnn_set_input_dense(spdnn_t *c, const float *y0, int batch, int first_glob
         rc = convert_dense_device(c, (const float *)c->stage, (int)rows, (int)(r0 / 32));
         if (rc) return rc;
     }
-    rc = repair_float_tiles(c);
-    if (rc) return rc;
+    if ((size_t)batch > chunk_rows) {
+        rc = repair_float_tiles(c);
+        if (rc) return rc;
+    }
     return end_input(c);
 }
 
@@ -1588,14 +1606,9 @@ int spdnn_sync(spdnn_t *c, spdnn_stats_t *stats) {
     if (!c) return SPDNN_ERR_ARG;
     DeviceGuard guard(c->device);
     if (c->in_flight) {
-        CK(cudaMemcpyAsync(c->host_ctl.data(), c->ctl, sizeof(LoopCtl) * (size_t)(c->nsteps + 1), cudaMemcpyDeviceToHost,
-                           c->stream));
-        CK(cudaMemcpyAsync(c->host_died.data(), c->died_at, sizeof(int32_t) * (size_t)c->layers, cudaMemcpyDeviceToHost,
-                           c->stream));
-        int32_t st = 0;
-        CK(cudaMemcpyAsync(&st, c->status, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         c->in_flight = false;
+        const int32_t st = *c->report.status;
         if (st != 0) {
             cudaMemsetAsync(c->status, 0, sizeof(int32_t), c->stream);
             return fail(c, SPDNN_ERR_DEVICE, "device-side check failed (code %d: %s)", st,
@@ -1605,11 +1618,11 @@ int spdnn_sync(spdnn_t *c, spdnn_stats_t *stats) {
         }
         spdnn_stats_t s{};
         s.layers = c->layers; s.batch = c->batch;
-        s.survivors = c->host_ctl[c->nsteps].live + c->host_ctl[c->nsteps].settled;
+        s.survivors = c->report.ctl[c->nsteps].live + c->report.ctl[c->nsteps].settled;
         {
             long long live = c->batch;
             for (int l = 0; l < c->layers; ++l) {
-                live -= c->host_died[l];
+                live -= c->report.died_at[l];
                 c->host_live[l] = (int32_t)live;
             }
             if (live != s.survivors) {
@@ -1626,7 +1639,7 @@ int spdnn_sync(spdnn_t *c, spdnn_stats_t *stats) {
             bytes += 4.0 * (c->n + 1) + 8.0 * (double)c->layer[l]->nnz;
         }
         s.algorithmic_bytes = bytes;
-        s.kernel_launches = c->nsteps + c->extra_launches + 1 + c->prep_launches;      // + finalize_ids_kernel
+        s.kernel_launches = c->nsteps + c->extra_launches + 1 + c->prep_launches;      // + finalize_kernel
         s.loop_launches = c->nsteps;
         s.resident_group = c->last_group;
         c->stats = s;
@@ -1655,14 +1668,12 @@ int spdnn_get_categories(spdnn_t *c, int32_t *ids, int capacity, int *count) {
     if (!c || !count) return SPDNN_ERR_ARG;
     if (c->in_flight) { int rc = spdnn_sync(c, nullptr); if (rc) return rc; }
     if (!c->result_ready) return fail(c, SPDNN_ERR_STATE, "no result: call spdnn_infer first");
-    const LoopCtl fin = c->host_ctl[c->nsteps];
+    const LoopCtl fin = c->report.ctl[c->nsteps];
     const int total = fin.live + fin.settled;
     *count = total;
     if (total == 0) return SPDNN_OK;
     if (!ids || capacity < total) return fail(c, SPDNN_ERR_ARG, "capacity %d < survivors %d", capacity, total);
-    DeviceGuard guard(c->device);
-    CK(cudaMemcpyAsync(ids, c->ids[fin.settled ? fin.ids_buf ^ 1 : fin.ids_buf], sizeof(int32_t) * (size_t)total, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    memcpy(ids, c->report.ids, sizeof(int32_t) * (size_t)total);
     return SPDNN_OK;
 }
 
@@ -1670,7 +1681,7 @@ int spdnn_get_activations(spdnn_t *c, float *y, int64_t capacity_rows) {
     if (!c) return SPDNN_ERR_ARG;
     if (c->in_flight) { int rc = spdnn_sync(c, nullptr); if (rc) return rc; }
     if (!c->result_ready) return fail(c, SPDNN_ERR_STATE, "no result: call spdnn_infer first");
-    const LoopCtl fin_ctl = c->host_ctl[c->nsteps];
+    const LoopCtl fin_ctl = c->report.ctl[c->nsteps];
     const int live = fin_ctl.live + fin_ctl.settled;
     if (live == 0) return SPDNN_OK;
     if (!y || capacity_rows < live) return fail(c, SPDNN_ERR_ARG, "capacity %lld < survivors %d", (long long)capacity_rows, live);
@@ -1684,7 +1695,7 @@ int spdnn_get_activations(spdnn_t *c, float *y, int64_t capacity_rows) {
     if (c->final_needs_expand) {
         // the last launch stored one row per class: copy it to the other members in every tile it wrote
         const DevRes &R = *c->res[c->final_expand_layer];
-        const int tiles = (c->host_ctl[c->nsteps - 1].live + 31) / 32;
+        const int tiles = (c->report.ctl[c->nsteps - 1].live + 31) / 32;
         const long long warps = (long long)tiles * R.classes;
         const int grid = (int)std::min<long long>((warps + 7) / 8, (long long)c->sm_count * 16);
         expand_members_kernel<<<std::max(1, grid), 256, 0, c->stream>>>(fin, c->tile_stride, tiles, R.mem_ptr, R.mem, R.classes);

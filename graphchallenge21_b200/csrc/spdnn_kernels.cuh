@@ -207,7 +207,7 @@ __device__ __forceinline__ float class_sum(const LayerDesc &d, int u, const floa
 // tiles 32 at a time with lane b handling bit b, so that the writes of the work list are
 // coalesced.  The global image numbers follow later and in parallel: when the order changed
 // (ids_buf flips) the blocks of the NEXT launch copy ids[ids_buf ^ 1][slot[j]] to ids[ids_buf][j]
-// for the images they own (move_id), and finalize_ids_kernel does it after the last launch.
+// for the images they own (move_id), and finalize_kernel does it after the last launch.
 __device__ __forceinline__ void rebuild_worklist(const LayerArgs &a, int live_in, int ids_buf) {
     __shared__ int s_warp[32];          // works for any block size up to 1024 threads
     __shared__ int s_total, s_settled;
@@ -463,19 +463,18 @@ static __global__ void tiles_to_dense_kernel(const float *__restrict__ y, long l
     }
 }
 
-// After the last launch of a pass that retired images (finalize_ids_kernel marked the images still on the work list in
-// `working`): lists the survivors, working or retired, in ascending order into ids[ids_buf ^ 1], and notes for each its
+// After the last launch of a pass that retired images (finalize_kernel marked the images still on the work list in
+// `working`): lists the survivors, working or retired, in ascending order into host_ids, and notes for each its
 // position in the work list (-1: retired).  A block takes kMergeWords words of the bitmaps and counts all words before
 // them itself (a few KB from L2), so that blocks need not wait for one another.
 constexpr int kMergeWords = 64;
-static __global__ void __launch_bounds__(256) merge_settled_kernel(const LoopCtl *ctl, int32_t *ids0, int32_t *ids1, const uint32_t *__restrict__ working,
+static __global__ void __launch_bounds__(256) merge_settled_kernel(const LoopCtl *ctl, const uint32_t *__restrict__ working,
                                                                    const uint32_t *__restrict__ settled, int words, const int32_t *first_id,
-                                                                   int32_t *work_of) {
+                                                                   int32_t *host_ids, int32_t *work_of) {
     __shared__ int s_all, s_work, s_cnt[2][kMergeWords];
     const LoopCtl c = *ctl;
     if (c.settled == 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = *first_id;
-    int32_t *to = c.ids_buf ? ids0 : ids1;
     const int q0 = blockIdx.x * kMergeWords, q1 = min(q0 + kMergeWords, words);
     if (tid == 0) s_all = s_work = 0;
     __syncthreads();
@@ -499,13 +498,12 @@ static __global__ void __launch_bounds__(256) merge_settled_kernel(const LoopCtl
         const uint32_t w = working[q], m = w | settled[q], below = (1u << lane) - 1u;
         if ((m >> lane) & 1u) {
             const int j = at + __popc(m & below);
-            to[j] = first + q * 32 + lane;
+            host_ids[j] = first + q * 32 + lane;
             work_of[j] = ((w >> lane) & 1u) ? wat + __popc(w & below) : -1;
         }
     }
 }
 
-// After the last launch: the ids of the final order, if that launch changed the order.
 // After a pass whose last launch stored one row per class (its first member): copy that row to the
 // other member rows of every tile the launch wrote, so that the tiles hold all N activations.
 // One warp per (tile, class), lane = image; mem[] holds member column * 32.
@@ -522,17 +520,30 @@ static __global__ void expand_members_kernel(float *__restrict__ y, long long ti
     }
 }
 
-static __global__ void finalize_ids_kernel(const LoopCtl *ctl, const int32_t *__restrict__ slot, int32_t *ids0, int32_t *ids1, uint32_t *working,
-                                           const int32_t *first_id) {
-    const LoopCtl c = *ctl;
-    if (c.identity && c.settled == 0) return;
+// The last launch of a pass: the ids of the final order, and everything the host asks for afterwards -- written straight
+// into page-locked host memory, so that fetching the results of a pass takes no copy and no second wait.
+struct HostReport {
+    int32_t *ids;                // [images] surviving image numbers (by merge_settled_kernel where images were retired)
+    LoopCtl *ctl;                // [nsteps + 1]
+    int32_t *died_at;            // [layers]
+    int32_t *status;
+};
+static __global__ void finalize_kernel(const LoopCtl *ctl0, int nsteps, const int32_t *__restrict__ slot, int32_t *ids0, int32_t *ids1,
+                                       const int32_t *__restrict__ died_at, int layers, const int32_t *status, const HostReport host,
+                                       uint32_t *working, const int32_t *first_id) {
+    const LoopCtl c = ctl0[nsteps];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     int32_t *ids = c.ids_buf ? ids1 : ids0;
     const int32_t *from = c.ids_buf ? ids0 : ids1;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < c.live; j += gridDim.x * blockDim.x) {
+    for (int j = t; j < c.live; j += step) {
         const int32_t id = c.identity ? ids[j] : __ldg(from + __ldg(slot + j));
         if (!c.identity) ids[j] = id;
-        if (c.settled) atomicOr(working + ((id - *first_id) >> 5), 1u << ((id - *first_id) & 31));
+        if (c.settled == 0) host.ids[j] = id;
+        else atomicOr(working + ((id - *first_id) >> 5), 1u << ((id - *first_id) & 31));
     }
+    for (int q = t; q < layers; q += step) host.died_at[q] = died_at[q];
+    for (int q = t; q <= nsteps; q += step) host.ctl[q] = ctl0[q];
+    if (t == 0) *host.status = *status;
 }
 
 // dense_cell: where the first launch of a pass finds the caller's row-major input when that launch
