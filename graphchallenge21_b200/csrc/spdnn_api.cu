@@ -375,9 +375,18 @@ int allow_max_dynamic_smem(spdnn *c, Kernel kernel) {
     return SPDNN_OK;
 }
 
+// Blocks of a launch whose blocks draw their groups of images: at most `groups`, at most what is on the device at once.
+template <typename Kernel>
+int drawing_grid(spdnn *c, Kernel kernel, int threads, size_t smem, int groups) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+    return std::max(1, std::min(groups, c->sm_count * per_sm));
+}
+
 template <int TI, int IPT, int KT, bool UNIFORM, bool STAGED>
 int launch_resident_t(spdnn *c, const ResArgs &a, int grid, size_t smem) {
     if (int rc = allow_max_dynamic_smem(c, resident_kernel<TI, IPT, KT, UNIFORM, STAGED>)) return rc;
+    if (!STAGED) grid = drawing_grid(c, resident_kernel<TI, IPT, KT, UNIFORM, STAGED>, SPDNN_GENERIC_THREADS, smem, grid);
     resident_kernel<TI, IPT, KT, UNIFORM, STAGED><<<grid, SPDNN_GENERIC_THREADS, smem, c->stream>>>(a);
     CK(cudaGetLastError());
     return SPDNN_OK;
@@ -418,7 +427,7 @@ template <int NT>
 int launch_inplace(spdnn *c, const ResArgs &a, int grid, size_t smem, bool k32, bool uniform) {
     auto go = [&](auto kernel) -> int {
         if (int rc = allow_max_dynamic_smem(c, kernel)) return rc;
-        kernel<<<grid, NT, smem, c->stream>>>(a);
+        kernel<<<drawing_grid(c, kernel, NT, smem, grid), NT, smem, c->stream>>>(a);
         CK(cudaGetLastError());
         return SPDNN_OK;
     };

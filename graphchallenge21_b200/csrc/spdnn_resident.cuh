@@ -183,6 +183,18 @@ __device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned int 
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
 
+// GENERIC chunk kernels that read their tables without barriers: the blocks that fit on the device at once draw groups of
+// images from an atomic counter (reset by the work-list rebuild), so that a launch most of whose images are gone -- the
+// groups are counted for all of them -- does not start thousands of blocks that do nothing (15000 blocks without an
+// image: 60 us, 296 that draw: 4).  A block's first group is its own number, which spreads few groups over the SMs; this returns
+// the next one.
+__device__ __forceinline__ int next_group(unsigned int *work, int *s_group) {
+    __syncthreads();                             // the block has left the group before
+    if (threadIdx.x == 0) *s_group = (int)atomicAdd(work, 1u);
+    __syncthreads();
+    return (int)gridDim.x + *s_group;
+}
+
 __device__ __forceinline__ void bulk_load_table(void *dst, const void *src, unsigned int bytes, unsigned long long *bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
@@ -357,8 +369,8 @@ __device__ __forceinline__ bool load_dense_rows(const float *dense, int n, int j
     return ns;
 }
 
-// Grid: one block per TI live images (launched for the worst case; surplus blocks only take
-// part in the last-block ticket).  Dynamic shared memory: two activation buffers of
+// Grid: STAGED one block per TI live images (launched for the worst case; surplus blocks only take
+// part in the last-block ticket), else the blocks that fit on the device, which take groups of TI (next_group).  Dynamic shared memory: two activation buffers of
 // buf_rows * TI * 4 bytes, then (STAGED) two table buffers of table_bytes each.
 // Threads per block: the GENERIC form is bound by shared-memory latency with one or two blocks
 // per SM (its buffers fill the shared memory), so it runs 16 warps.
@@ -376,7 +388,7 @@ resident_kernel(const ResArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned int s_alive[3];
     __shared__ unsigned int s_open[3];           // images with an output of layer li % 3 that is not clip
-    __shared__ int s_last, s_fail;
+    __shared__ int s_last, s_fail, s_group;
     __shared__ __align__(8) unsigned long long s_bar[2];
     if (a.gate != nullptr && *a.gate != a.gate_want) return;
     constexpr int NQ = IPT / 4;                  // float4 halves per thread
@@ -391,12 +403,13 @@ resident_kernel(const ResArgs a) {
     const int nblk = (live_in + TI - 1) / TI;
     const int buf_bytes = a.buf_rows * RS;
 
-    // a tile that the count_kernel pre-pass finished is skipped (TI divides 32: a block lies inside one tile)
-    const bool tile_finished = a.tile_done != nullptr && (int)blockIdx.x < nblk && a.tile_done[(blockIdx.x * TI) >> 5] != 0;
-    if ((int)blockIdx.x < nblk && !tile_finished) {
+    // STAGED: one group per block, whose barriers serve once
+    for (int group = blockIdx.x; group < nblk; group = STAGED ? nblk : next_group(a.work, &s_group)) {
+        // a tile that the count_kernel pre-pass finished is skipped (TI divides 32: a group lies inside one tile)
+        if (a.tile_done != nullptr && a.tile_done[(group * TI) >> 5] != 0) continue;
         unsigned char *cur = smem, *nxt = smem + buf_bytes;
         unsigned char *const tbl0 = smem + 2 * buf_bytes;      // table buffer q sits at tbl0 + q * table_bytes
-        const int j0 = blockIdx.x * TI;
+        const int j0 = group * TI;
         if (tid == 0) {
             s_alive[0] = s_open[0] = 0u;
             s_fail = 0;
@@ -668,15 +681,15 @@ __global__ void __launch_bounds__(NT, 1024 / NT) inplace_kernel(const ResArgs a)
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned int s_alive[3];
     __shared__ unsigned int s_open[3];           // images with an output of layer li % 3 that is not clip
-    __shared__ int s_last;
+    __shared__ int s_last, s_group;
     constexpr int RS = 128, CPP = NT / 8;        // bytes per row; classes per pass of the block
     if (a.gate != nullptr && *a.gate != a.gate_want) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int sub = tid & 7, grp = tid >> 3;
     const LoopCtl ctl = *a.ctl_in;
-    const int live_in = ctl.live, tile = blockIdx.x;
-    const bool tile_finished = a.tile_done != nullptr && tile * 32 < live_in && a.tile_done[tile] != 0;
-    if (tile * 32 < live_in && !tile_finished) {
+    const int live_in = ctl.live;
+    for (int tile = blockIdx.x; tile < (live_in + 31) / 32; tile = next_group(a.work, &s_group)) {
+        if (a.tile_done != nullptr && a.tile_done[tile] != 0) continue;
         const bool valid = tile * 32 + lane < live_in;
         {
             // one row per value id: a lane owns an image, a warp a row; up to UNR loads in flight
