@@ -593,6 +593,8 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
     int resident_chunks = 0;       // resident chunks planned so far
     int alt2_chunks = 0;           // ALT2 chunks planned so far
     int generic_chunks = 0;        // GENERIC chunks planned so far
+    bool split = false;            // the first ALT2 chunk was split in two (see below)
+    const bool own_lengths = c->chunk_list.empty() && !c->chunk_growth_set && c->chunk_first == 8;
     int short_chunk = 0;           // > 0: `chunk` was raised to the rest of the network at once; the length it would have had
     while (l < c->layers) {
         Step st;
@@ -643,6 +645,14 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
             if (ti) {
                 // extend while the layers are of one kernel variant and the group still fits
                 int f = 1, blob = R0.blob_bytes, maxc = R0.classes;
+                if (R0.mode == kResAlt2 && alt2_chunks == 0 && chunk == 8 && own_lengths) {
+                    // Blocks that fill an SM and many of them: two thirds of the images die within the first eight layers, and the
+                    // second four without the dead cost less than the launch between (16384 neurons, layer loop: 60000 images
+                    // 1703 -> 1617 us, 6000 images 298 -> 317).
+                    split = ti == 16 && resident_smem_bytes(ti, rows, 0) * 2 + 4096 > (size_t)c->smem_optin &&
+                            (long long)c->tiles_cap * 32 >= 16LL * 8 * c->sm_count;
+                    if (split) chunk = 4;
+                }
                 while (f < chunk && l + f < c->layers && c->res[l + f]) {
                     const DevRes &M = *c->res[l + f];
                     if (M.mode != R0.mode || M.uniform != R0.uniform || (M.k == 32) != k32) break;
@@ -703,7 +713,7 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                     // tile that is not saturated costs the pre-pass a read of all its rows for nothing.
                     const int rows_max = std::max(rows, maxc);
                     if (c->bits_prepass && c->bit_form && c->clip > 0.0f && (maxc > 64 || c->bits_small) && rows_max <= 16383 &&
-                        (alt2_chunks > 1 || c->bits_first_chunk)) {
+                        ((alt2_chunks > 1 && l > 12) || c->bits_first_chunk)) {
                         st.wwords = (rows_max + 63) / 64 * 64;
                         const int passes = (maxc + 63) / 64;
                         int nt = c->bits_threads > 0 ? c->bits_threads : 32 * ((passes + 1) / 2);
@@ -750,16 +760,19 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
             if (resident_chunks < (int)c->chunk_list.size()) chunk = c->chunk_list[resident_chunks];
             else {
                 const bool alt2 = st.max_classes > 0;
+                const int nth = alt2_chunks - (split ? 1 : 0);
                 const bool prepass = alt2 && (st.max_classes > 64 || c->bits_small) && c->bits_prepass && c->bit_form && c->clip > 0.0f;
                 short_chunk = 0;
-                if (prepass && alt2_chunks >= 1 && !c->chunk_growth_set) {
+                if (alt2 && split && alt2_chunks < 2) {
+                    chunk = alt2_chunks == 0 ? 4 : 32;
+                } else if (prepass && nth >= 1 && !c->chunk_growth_set) {
                     // A chunk with a bits_kernel pre-pass runs its saturated tiles at a fraction of the float form's cost
                     // and dead images cost it nothing, so such chunks can be long.  But a tile that is NOT saturated when
                     // the chunk starts is alt2_kernel's for the whole chunk (at 65536 neurons about 1.4 us per layer and
                     // tile against 0.3): the first chunk with a pre-pass is as short as the chunk before it, and only the
                     // one after it takes the rest of the network -- a tile that saturates a few layers late then costs
                     // tens of layers, not thousands (measured: one such tile among 7500 images made a pass 2.6 ms longer).
-                    if (alt2_chunks >= 2) chunk = c->chunk_max;
+                    if (nth >= 2) chunk = c->chunk_max;
                 } else {
                     chunk = std::min(chunk * (alt2 ? c->chunk_growth : c->chunk_growth_generic), c->chunk_max);
                     // Images without structure saturate one by one soon after the first chunk, at clip everywhere, and leave the
@@ -774,7 +787,7 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                 // Where the tables repeat, alt2_kernel's own bit form ends a tile one period after it saturates
                 // (ResArgs::period): from the third ALT2 chunk on one launch takes the rest of the network, provided that
                 // its word ring has room for a period (checked when the chunk is planned).
-                if (alt2 && alt2_chunks == 1 && c->fixed_point && c->bit_form && !c->chunk_growth_set && chunk < c->chunk_max) {
+                if (alt2 && nth == 1 && c->fixed_point && c->bit_form && !c->chunk_growth_set && chunk < c->chunk_max) {
                     short_chunk = chunk;
                     chunk = c->chunk_max;
                 }
