@@ -120,15 +120,23 @@ inline std::string canonicalize_layer(int n, const int32_t *col_ptr, const int32
 // Whether the layer maps the vector whose every entry is `clip` onto itself: each column's sum, added and rounded as the
 // kernels do it, reaches clip with the bias.  (Every product and sum is rounded to fp32 by its store.)
 inline bool keeps_top(const HostLayer &h, float bias, float clip) {
+    std::vector<signed char> of_count(h.k + 1, -1);      // uniform weight: the sum depends on the number of entries alone
     for (int c = 0; c < h.n; ++c) {
         const int32_t *r = &h.rows[(size_t)c * h.k];
+        int count = h.k;                                  // padding (rows past the last neuron) is at the end
+        while (count > 0 && r[count - 1] >= h.n) --count;
+        if (h.uniform && of_count[count] >= 0) {
+            if (!of_count[count]) return false;
+            continue;
+        }
         volatile float sum = 0.0f;
-        for (int i = 0; i < h.k && r[i] < h.n; ++i) {
+        for (int i = 0; i < count; ++i) {
             volatile float term = h.uniform ? clip : clip * h.vals[(size_t)c * h.k + i];
             sum = sum + term;
         }
         volatile float y = h.uniform ? sum * h.w : sum;
         y = y + bias;
+        of_count[count] = y >= clip;
         if (!(y >= clip)) return false;
     }
     return true;

@@ -221,8 +221,9 @@ int free_buffers(spdnn *c) {
     c->open_mask = c->settled = c->working = nullptr; c->work_of = nullptr;
     c->y[0] = c->y[1] = nullptr; c->slot = nullptr; c->mask = nullptr; c->ids[0] = c->ids[1] = nullptr;
     c->tile_done = nullptr; c->xw = nullptr; c->has_floats = nullptr; c->in_flag = nullptr;
-    cudaFreeHost(c->report.ids);
-    c->report.ids = nullptr;
+    cudaFreeHost(c->report.ctl);
+    c->report = HostReport{};
+    c->result_ready = c->input_ready = false;      // (their memory is gone)
     c->tiles_cap = 0;
     return SPDNN_OK;
 }
@@ -239,7 +240,16 @@ int ensure_capacity(spdnn *c, int batch) {
         CK(cudaMemsetAsync(c->y[i], 0, ybytes, c->stream));      // incl. the permanent zero row of every tile
         CK(cudaMalloc(&c->ids[i], sizeof(int32_t) * (size_t)tiles * 32));
     }
-    CK(cudaMallocHost(&c->report.ids, sizeof(int32_t) * (size_t)tiles * 32));
+    {
+        // one block: the records per launch boundary, the deaths per layer, the status, the image numbers
+        unsigned char *block = nullptr;
+        const size_t ctl_bytes = sizeof(LoopCtl) * (size_t)(c->layers + 1);
+        CK(cudaMallocHost(&block, ctl_bytes + sizeof(int32_t) * ((size_t)c->layers + 1 + (size_t)tiles * 32)));
+        c->report.ctl = reinterpret_cast<LoopCtl *>(block);
+        c->report.died_at = reinterpret_cast<int32_t *>(block + ctl_bytes);
+        c->report.status = c->report.died_at + c->layers;
+        c->report.ids = c->report.status + 1;
+    }
     CK(cudaMalloc(&c->slot, sizeof(int32_t) * (size_t)tiles * 32));
     CK(cudaMalloc(&c->mask, sizeof(uint32_t) * (size_t)tiles));
     CK(cudaMemsetAsync(c->mask, 0, sizeof(uint32_t) * (size_t)tiles, c->stream));
@@ -764,7 +774,7 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                 const bool prepass = alt2 && (st.max_classes > 64 || c->bits_small) && c->bits_prepass && c->bit_form && c->clip > 0.0f;
                 short_chunk = 0;
                 if (alt2 && split && alt2_chunks < 2) {
-                    chunk = alt2_chunks == 0 ? 4 : 32;
+                    chunk = std::min(alt2_chunks == 0 ? 4 : 32, c->chunk_max);
                 } else if (prepass && nth >= 1 && !c->chunk_growth_set) {
                     // A chunk with a bits_kernel pre-pass runs its saturated tiles at a fraction of the float form's cost
                     // and dead images cost it nothing, so such chunks can be long.  But a tile that is NOT saturated when
@@ -1202,16 +1212,6 @@ int spdnn_create(spdnn_t **out, int device, int neurons, int layers, float bias,
     CK(cudaMalloc(&c->died_at, sizeof(int32_t) * (size_t)layers));
     CK(cudaMemset(c->died_at, 0, sizeof(int32_t) * (size_t)layers));
     CK(cudaMalloc(&c->res_table, sizeof(ResLayer) * (size_t)layers));
-    {
-        // one block: the records per launch boundary, the deaths per layer, the status
-        unsigned char *block = nullptr;
-        const size_t ctl_bytes = sizeof(LoopCtl) * (size_t)(layers + 1);
-        CK(cudaMallocHost(&block, ctl_bytes + sizeof(int32_t) * ((size_t)layers + 1)));
-        memset(block, 0, ctl_bytes + sizeof(int32_t) * ((size_t)layers + 1));
-        c->report.ctl = reinterpret_cast<LoopCtl *>(block);
-        c->report.died_at = reinterpret_cast<int32_t *>(block + ctl_bytes);
-        c->report.status = c->report.died_at + layers;
-    }
     c->host_live.assign(layers, 0);
     {
         int optin = 0;
@@ -1275,7 +1275,6 @@ void spdnn_destroy(spdnn_t *c) {
     for (int kind = 0; kind < 2; ++kind)
         if (c->graph_exec[kind]) cudaGraphExecDestroy(c->graph_exec[kind]);
     cudaFree(c->dense_cell); cudaFree(c->first_cell);
-    cudaFreeHost(c->report.ctl);
     free_buffers(c);
     cudaFree(c->ctl); cudaFree(c->counter); cudaFree(c->status); cudaFree(c->stage);
     cudaFree(c->died_at); cudaFree(c->res_table);
