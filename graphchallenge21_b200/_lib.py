@@ -40,6 +40,7 @@ SYMBOLS = {
     "spdnn_get_layer_live": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int]),
     "spdnn_get_categories": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_int)]),
     "spdnn_get_activations": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64]),
+    "spdnn_get_shortcuts": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     "spdnn_get_layer_info": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "spdnn_inspect_layer_csc": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int),
                                           C.POINTER(C.c_int)]),

@@ -302,7 +302,9 @@ alt2_kernel(const ResArgs a) {
                     int waited_group = -1;                   // the group of tables these threads have seen arrive
                     unsigned int tt_cur = 0xffffffffu;       // no truth table has this value
                     TruthMasks tm = truth_masks(0u);
-                    bool first_period = true;                // the first periodic group is one period, so that a fixed point shows early
+                    const int ring_periods = a.period > 0 ? (a.wring - 1) / a.period : 0;
+                    int watch_left = 0, watch_from = 0;      // layers left of the periods watched (0: none), their first word buffer
+                    bool first_watch = true;
                     while (li < nl) {
                         if (STAGED && (li >> gshift) != waited_group) {
                             if (leader) issue_groups(li);
@@ -314,15 +316,22 @@ alt2_kernel(const ResArgs a) {
                             }
                             waited_group = li >> gshift;
                         }
+                        // Fixed point: watch whole periods of the chunk's tables from here (first one, so that it shows early, then
+                        // as many as the ring of word buffers can hold without overwriting the buffer they start from).  A
+                        // period may take several groups, for a table copy can bring fewer layers than it has.
+                        if (watch_left == 0 && careful == 0 && ring_periods > 0 && li >= a.period_from) {
+                            int len = first_watch ? a.period : ring_periods * a.period;
+                            if (li + len >= nl) len = a.period;
+                            if (li + len < nl) {
+                                watch_left = len;
+                                watch_from = ws;
+                                first_watch = false;
+                            }
+                        }
                         int cnt = min(a.wring - 1, nl - li);
                         if (STAGED) cnt = min(cnt, (1 << gshift) - (li & gmask));
+                        if (watch_left > 0) cnt = min(cnt, watch_left);
                         if (careful > 0) cnt = 1;
-                        // whole periods of the chunk's tables where one fits (see below: fixed point)
-                        bool periodic = a.period > 0 && li >= a.period_from && cnt >= a.period;
-                        if (periodic) {
-                            cnt = first_period ? a.period : cnt / a.period * a.period;
-                            first_period = false;
-                        }
                         const unsigned char *T = table_of(li);
                         // The layers of a group are applied with one truth table: lane g looks at layer g's, and
                         // a group whose layers differ (another K or weight) is cut down to its first layer.
@@ -331,7 +340,7 @@ alt2_kernel(const ResArgs a) {
                             const unsigned int tl = STAGED ? *reinterpret_cast<const unsigned int *>(hp) : __ldg(reinterpret_cast<const unsigned int *>(hp));
                             const unsigned int t0 = __shfl_sync(0xffffffffu, tl, 0);
                             const bool same = multi ? __syncthreads_and(tl == t0 ? 1 : 0) != 0 : __all_sync(0xffffffffu, tl == t0);
-                            if (!same) { cnt = 1; periodic = false; }
+                            if (!same) cnt = 1;
                             if (t0 != tt_cur) {
                                 tt_cur = t0;
                                 tm = truth_masks(t0);
@@ -426,23 +435,30 @@ alt2_kernel(const ResArgs a) {
                         if (ns_any != 0u || (now != alive && cnt > 1)) {
                             if (cnt == 1) break;         // layer li has an unsaturated output: the float form applies it
                             careful = cnt;               // repeat the group from its first buffer, layer by layer
+                            watch_left = 0;
                             continue;
                         }
-                        if (now != alive && leader) atomicAdd(a.died_at + li, __popc(alive & ~now));     // cnt == 1
+                        if (now != alive) {              // cnt == 1
+                            if (leader) atomicAdd(a.died_at + li, __popc(alive & ~now));
+                            watch_left = 0;
+                        }
                         alive = now;
                         li += cnt;
                         done_classes = classes;
-                        if (periodic && li < nl) {
-                            // Fixed point: the tables repeat with this period and the group's last words are those it
-                            // started from (its first buffer is still intact), so every later whole period changes
-                            // nothing -- no image dies in one and no output is unsaturated, as none was in this one --
-                            // and only the layers behind the last whole period are left.  They use the tables of the
-                            // layers that follow here.  (1024 neurons, layers 41 .. 1919 of 60000 images: 239 -> 15 us.)
-                            const unsigned int *w0 = wring0 + (size_t)ws * a.rows_w, *w1 = wring0 + (size_t)s * a.rows_w;
+                        if (watch_left > 0 && (watch_left -= cnt) == 0) {
+                            // The tables repeat with this period and the last words are those the watched layers started
+                            // from: every later whole period changes nothing -- no image dies in one and no output is
+                            // unsaturated, as none was in these -- and only the layers behind the last whole period are
+                            // left.  They use the tables of the layers that follow here.  (1024 neurons, layers 41 .. 1919
+                            // of 60000 images: 239 -> 15 us.)
+                            const unsigned int *w0 = wring0 + (size_t)watch_from * a.rows_w, *w1 = wring0 + (size_t)s * a.rows_w;
                             unsigned int moved = 0u;
                             for (int q = multi ? tid : lane; q < classes; q += multi ? NT : 32) moved |= w0[q] ^ w1[q];
-                            if (multi ? !__syncthreads_or(moved != 0u ? 1 : 0) : __all_sync(0xffffffffu, moved == 0u))
-                                nl = li + (nl - li) % a.period;
+                            if (multi ? !__syncthreads_or(moved != 0u ? 1 : 0) : __all_sync(0xffffffffu, moved == 0u)) {
+                                const int end = li + (nl - li) % a.period;
+                                if (leader) atomicAdd(a.skipped, (unsigned int)(nl - end));
+                                nl = end;
+                            }
                         }
                         ws = s;
                         if (careful > 0) --careful;

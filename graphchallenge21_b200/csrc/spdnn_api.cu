@@ -158,7 +158,7 @@ struct spdnn {
     int extra_launches = 0;            // pre-pass launches of the captured schedule
     int graph_extra[2] = {0, 0};
     int32_t *ids[2] = {nullptr, nullptr};
-    unsigned int *counter = nullptr;   // [0] blocks finished, [1] next work item, [2] images retired by a launch
+    unsigned int *counter = nullptr;   // [0] blocks finished, [1] next work item, [2] images retired by a launch, [3] layers skipped in this pass
     int32_t *status = nullptr;
 
     void *stage = nullptr;             // device staging for host inputs / outputs
@@ -241,14 +241,15 @@ int ensure_capacity(spdnn *c, int batch) {
         CK(cudaMalloc(&c->ids[i], sizeof(int32_t) * (size_t)tiles * 32));
     }
     {
-        // one block: the records per launch boundary, the deaths per layer, the status, the image numbers
+        // one block: the records per launch boundary, the deaths per layer, the status, the layers skipped, the image numbers
         unsigned char *block = nullptr;
         const size_t ctl_bytes = sizeof(LoopCtl) * (size_t)(c->layers + 1);
-        CK(cudaMallocHost(&block, ctl_bytes + sizeof(int32_t) * ((size_t)c->layers + 1 + (size_t)tiles * 32)));
+        CK(cudaMallocHost(&block, ctl_bytes + sizeof(int32_t) * ((size_t)c->layers + 2 + (size_t)tiles * 32)));
         c->report.ctl = reinterpret_cast<LoopCtl *>(block);
         c->report.died_at = reinterpret_cast<int32_t *>(block + ctl_bytes);
         c->report.status = c->report.died_at + c->layers;
-        c->report.ids = c->report.status + 1;
+        c->report.skipped = reinterpret_cast<uint32_t *>(c->report.status + 1);
+        c->report.ids = c->report.status + 2;
     }
     CK(cudaMalloc(&c->slot, sizeof(int32_t) * (size_t)tiles * 32));
     CK(cudaMalloc(&c->mask, sizeof(uint32_t) * (size_t)tiles));
@@ -320,7 +321,8 @@ int repair_float_tiles(spdnn *c) {
 
 int end_input(spdnn *c) {
     init_loop_kernel<<<std::max(1, std::min(1024, (c->batch + 255) / 256)), 256, 0, c->stream>>>(
-        c->ctl, c->ids[0], c->batch, c->first_id, c->died_at, c->layers, c->dense_cell, c->dense_src, c->first_cell, c->settled, c->working, c->tiles_cap);
+        c->ctl, c->ids[0], c->batch, c->first_id, c->died_at, c->layers, c->dense_cell, c->dense_src, c->first_cell, c->settled, c->working, c->tiles_cap,
+        c->counter + 3);
     CK(cudaGetLastError());
     c->prep_launches += 1;
     CK(cudaEventRecord(c->ev_prep1, c->stream));
@@ -703,12 +705,6 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                         return alt2_smem_bytes(t_i, rows, st.stride, st.gshift, st.tring);
                     };
                     const size_t need = stage(ti, (size_t)c->smem_optin);
-                    if (short_chunk > 0 && !(st.period > 0 && st.period < st.wring)) {
-                        // no fixed point to look for, or no room to look for it: grow step by step (see below)
-                        chunk = short_chunk;
-                        short_chunk = 0;
-                        continue;
-                    }
                     // A block that has an SM to itself cannot hide the loading and storing of its rows, nor the tail of a
                     // layer, behind another block's arithmetic: where half the images per block (and tables staged at
                     // least four layers at a time) let two blocks share an SM, that is faster (measured at 16384 neurons).
@@ -716,6 +712,12 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                         const size_t half = stage(ti / 2, ((size_t)c->smem_optin - 4096) / 2);
                         if (st.tring > 0 && st.gshift >= 2 && half * 2 + 4096 <= (size_t)c->smem_optin) ti /= 2;
                         else stage(ti, (size_t)c->smem_optin);
+                    }
+                    if (short_chunk > 0 && !(st.period > 0 && st.period < st.wring)) {
+                        // no fixed point to look for, or no room in the ring to look for it: grow step by step (see below)
+                        chunk = short_chunk;
+                        short_chunk = 0;
+                        continue;
                     }
                     // Pre-pass for tiles that are saturated already (bits_kernel): layers of more than one pass of 64
                     // classes, where the float buffers leave this kernel's own bit form few images per block.  Not
@@ -796,7 +798,9 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                 }
                 // Where the tables repeat, alt2_kernel's own bit form ends a tile one period after it saturates
                 // (ResArgs::period): from the third ALT2 chunk on one launch takes the rest of the network, provided that
-                // its word ring has room for a period (checked when the chunk is planned).
+                // its word ring has room for a period (checked when the chunk is planned; a table copy may be shorter).  A tile that
+                // saturates in that launch then ends a period later (16384 neurons, 1920 layers, 64 images, one of them
+                // saturating at layer 65: 1176 us, against 2016 where periods had to lie inside one table copy of four layers).
                 if (alt2 && nth == 1 && c->fixed_point && c->bit_form && !c->chunk_growth_set && chunk < c->chunk_max) {
                     short_chunk = chunk;
                     chunk = c->chunk_max;
@@ -892,7 +896,7 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
             a.bit_ok = (alt2 && c->bit_form && c->clip > 0.0f && st.wring >= 2) ? 1 : 0;
             a.tile_done = nullptr; a.wwords = 0;
             a.cache = nullptr; a.rec_of = nullptr; a.cache_records = 0;
-            a.period = st.period; a.period_from = st.period_from;
+            a.period = st.period; a.period_from = st.period_from; a.skipped = c->counter + 3;
             a.gate = nullptr; a.gate_want = 0;
             a.xw = step == 0 && front == kFrontInPlace ? c->xw : nullptr;
             a.xw_flag = c->in_flag; a.nw = c->nw;
@@ -1040,7 +1044,7 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
     }
     c->nsteps = (int)plan.size();
     finalize_kernel<<<std::max(1, std::min(c->tiles_cap, 4 * c->sm_count)), 256, 0, c->stream>>>(
-        c->ctl, c->nsteps, c->slot, c->ids[0], c->ids[1], c->died_at, c->layers, c->status, c->report, c->working,
+        c->ctl, c->nsteps, c->slot, c->ids[0], c->ids[1], c->died_at, c->layers, c->status, c->counter + 3, c->report, c->working,
         c->first_cell);
     CK(cudaGetLastError());
     if (c->retires) {
@@ -1202,8 +1206,8 @@ int spdnn_create(spdnn_t **out, int device, int neurons, int layers, float bias,
     c->layer.resize(layers);
     CK(cudaMalloc(&c->ctl, sizeof(LoopCtl) * (size_t)(layers + 1)));
     CK(cudaMemset(c->ctl, 0, sizeof(LoopCtl) * (size_t)(layers + 1)));
-    CK(cudaMalloc(&c->counter, 3 * sizeof(unsigned int)));
-    CK(cudaMemset(c->counter, 0, 3 * sizeof(unsigned int)));
+    CK(cudaMalloc(&c->counter, 4 * sizeof(unsigned int)));
+    CK(cudaMemset(c->counter, 0, 4 * sizeof(unsigned int)));
     CK(cudaMalloc(&c->status, sizeof(int32_t)));
     CK(cudaMalloc(&c->first_cell, sizeof(int32_t)));
     CK(cudaMalloc(&c->dense_cell, sizeof(const float *)));
@@ -1734,6 +1738,15 @@ int spdnn_get_activations(spdnn_t *c, float *y, int64_t capacity_rows) {
         CK(cudaMemcpyAsync(y + r0 * c->n, c->stage, rows * row_bytes, cudaMemcpyDeviceToHost, c->stream));
     }
     CK(cudaStreamSynchronize(c->stream));
+    return SPDNN_OK;
+}
+
+int spdnn_get_shortcuts(spdnn_t *c, int64_t *retired_images, int64_t *skipped_layers) {
+    if (!c) return SPDNN_ERR_ARG;
+    if (c->in_flight) { int rc = spdnn_sync(c, nullptr); if (rc) return rc; }
+    if (!c->result_ready) return fail(c, SPDNN_ERR_STATE, "no result: call spdnn_infer first");
+    if (retired_images) *retired_images = c->report.ctl[c->nsteps].settled;
+    if (skipped_layers) *skipped_layers = *c->report.skipped;
     return SPDNN_OK;
 }
 

@@ -309,7 +309,11 @@ __global__ void __launch_bounds__(kBitsMaxThreads, 1) bits_kernel(const ResArgs 
                 const bool fixed = !__syncthreads_or(moved != 0u ? 1 : 0) && periodic;      // (everyone has read s_or[0])
                 if (tid == 0) s_or[0] = s_or[1] = s_or[2] = 0u;
                 if (any_ns) { unsat = true; break; }
-                if (fixed) nl = li + (nl - li) % period;       // (nobody died: a dead image's words were not all zero before)
+                if (fixed) {                                   // (nobody died: a dead image's words were not all zero before)
+                    const int end = li + (nl - li) % period;
+                    if (tid == 0) atomicAdd(a.skipped, (unsigned int)(nl - end));
+                    nl = end;
+                }
                 if (now != alive) {
                     // somebody died inside the segment: again from its input, layer by layer (the tracked loop wants
                     // its three slots zero and leaves them in any state)

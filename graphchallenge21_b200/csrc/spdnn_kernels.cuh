@@ -527,9 +527,10 @@ struct HostReport {
     LoopCtl *ctl;                // [nsteps + 1]
     int32_t *died_at;            // [layers]
     int32_t *status;
+    uint32_t *skipped;           // layers the blocks did not apply because their words had settled
 };
 static __global__ void finalize_kernel(const LoopCtl *ctl0, int nsteps, const int32_t *__restrict__ slot, int32_t *ids0, int32_t *ids1,
-                                       const int32_t *__restrict__ died_at, int layers, const int32_t *status, const HostReport host,
+                                       const int32_t *__restrict__ died_at, int layers, const int32_t *status, const unsigned int *skipped, const HostReport host,
                                        uint32_t *working, const int32_t *first_id) {
     const LoopCtl c = ctl0[nsteps];
     const int t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
@@ -543,14 +544,14 @@ static __global__ void finalize_kernel(const LoopCtl *ctl0, int nsteps, const in
     }
     for (int q = t; q < layers; q += step) host.died_at[q] = died_at[q];
     for (int q = t; q <= nsteps; q += step) host.ctl[q] = ctl0[q];
-    if (t == 0) *host.status = *status;
+    if (t == 0) { *host.status = *status; *host.skipped = *skipped; }
 }
 
 // dense_cell: where the first launch of a pass finds the caller's row-major input when that launch
 // reads it in place (dense_src, may be null: the input was converted to tiles).
 static __global__ void init_loop_kernel(LoopCtl *ctl, int32_t *ids0, int batch, int first_global_id, int32_t *died_at,
                                         int layers, const float **dense_cell, const float *dense_src, int32_t *first_cell,
-                                        uint32_t *settled, uint32_t *working, int words) {
+                                        uint32_t *settled, uint32_t *working, int words, unsigned int *skipped) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x)
         ids0[i] = first_global_id + i;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < layers; i += gridDim.x * blockDim.x) died_at[i] = 0;
@@ -560,6 +561,7 @@ static __global__ void init_loop_kernel(LoopCtl *ctl, int32_t *ids0, int batch, 
         c.live = batch; c.identity = 1; c.ids_buf = 0; c.settled = 0;
         *ctl = c;
         *first_cell = first_global_id;
+        *skipped = 0u;
         *dense_cell = dense_src;
     }
 }

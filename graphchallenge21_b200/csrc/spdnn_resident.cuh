@@ -104,6 +104,7 @@ struct ResArgs {
     // The chunk's tables repeat: layer q + period uses the tables of layer q for every q >= period_from (0: no period).
     // Saturated activations that one period maps onto themselves are then a fixed point of all later periods.
     int period, period_from;
+    unsigned int *skipped;    // layers not applied because a block's words had settled, summed over the blocks of a pass
     // First chunk of a pass, GENERIC tables: where *xw_flag is 0 the input is binary and is read from its words (bit i of
     // xw[tile * nw + r] = image i of the tile has neuron r set) instead of the float tiles; nullptr: float tiles
     const uint32_t *xw;

@@ -240,6 +240,12 @@ class SpDNN:
         self._check(self._lib.spdnn_get_activations(self._ctx, _ptr(y) if count else None, count))
         return y
 
+    def shortcuts(self) -> dict:
+        """What the last pass left out (``spdnn_get_shortcuts``): images retired at clip, layers behind fixed points."""
+        retired, skipped = C.c_int64(), C.c_int64()
+        self._check(self._lib.spdnn_get_shortcuts(self._ctx, C.byref(retired), C.byref(skipped)))
+        return {"retired_images": retired.value, "skipped_layers": skipped.value}
+
 
 def pack_bits(y0: np.ndarray) -> np.ndarray:
     """[batch, N] array -> the bit matrix ``set_input_bits`` takes (non-zero = 1), rows padded to whole 32-bit words."""

@@ -147,6 +147,12 @@ int spdnn_get_categories(spdnn_t *ctx, int32_t *ids, int capacity, int *count);
  * order of spdnn_get_categories (the reference copies C back at all_network.cu:521). */
 int spdnn_get_activations(spdnn_t *ctx, float *y, int64_t capacity_rows);
 
+/* What the last pass left out because it could not change the result: retired_images = survivors taken off the
+ * work list once every activation was clip and every later layer keeps that; skipped_layers = layers of periodic
+ * networks behind a fixed point of the saturated activations, summed over the blocks that found one.  For tests
+ * and for judging a schedule; either pointer may be NULL. */
+int spdnn_get_shortcuts(spdnn_t *ctx, int64_t *retired_images, int64_t *skipped_layers);
+
 /* How the library stored layer `layer`: classes = number of distinct columns (columns with
  * identical rows and weights are computed once), k = padded non-zeros per column,
  * uniform = 1 when all weights are one power-of-two constant.  Any pointer may be NULL. */
