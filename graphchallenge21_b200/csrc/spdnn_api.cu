@@ -73,6 +73,9 @@ struct DevRes {
     }
 };
 
+// The last resident step of a schedule runs in groups of ti when it finds at most `images` images (ti == 0: never).
+struct SmallGroups { int step = 0, ti = 0, images = 0; };
+
 }  // namespace
 
 struct spdnn {
@@ -117,6 +120,7 @@ struct spdnn {
     int res_ti_max = 32;               // largest group of images per block to try
     int res_ipt_max = 8;               // most images per thread to try
     int last_group = 0;                // group size of the last captured schedule's resident launches
+    SmallGroups last_small;            // ... and the smaller one its last resident step may have run in instead
     int smem_optin = 0;                // shared memory one block may opt in to
     bool stage_tables = true;          // bring the per-layer tables into shared memory with bulk copies
     int chunk_first = 8, chunk_max = 2048, chunk_growth = 4;      // SPDNN_CHUNK_FIRST / _MAX / _GROWTH
@@ -171,6 +175,7 @@ struct spdnn {
     // caller's row-major matrix in place (only when that launch is a resident chunk; else null).
     cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
     int graph_steps[2] = {0, 0}, graph_group[2] = {0, 0};
+    SmallGroups graph_small[2];
     bool graph_dirty = true;
     bool alt2_small_blocks = true;     // SPDNN_ALT2_SMALL_BLOCKS=0: 256-thread blocks also for layers of <= 64 classes
     bool lazy_expand = true;           // SPDNN_LAZY_EXPAND=0: the last launch of a pass writes all member rows itself
@@ -577,6 +582,8 @@ struct Step {
     unsigned char *cache = nullptr;
     unsigned short *rec_of = nullptr;
     int cache_records = 0;
+    // GENERIC chunk: groups of small_ti images instead when at most small_images are on the work list (0: no such launch)
+    int small_ti = 0, small_table = 0, small_images = 0;
     int period = 0, period_from = 0;      // ALT2 chunk: its tables repeat with this period from this layer of the chunk on (0: no)
 };
 
@@ -628,13 +635,10 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
             const int (*cand)[2] = R0.mode == kResAlt2 ? kAlt2 : kGeneric;
             const int ncand = R0.mode == kResAlt2 ? 5 : 4;
             // GENERIC groups: as many images as still give every SM a block; a block's time grows with its images, so a
-            // small batch is faster in smaller groups on more SMs ...
+            // small batch is faster in smaller groups on more SMs
             int most = 32;
-            if (R0.mode == kResGeneric) {
+            if (R0.mode == kResGeneric)
                 while (most > 4 && c->tiles_cap * (32 / most) < c->sm_count) most /= 2;
-                // ... and so are the few images that are left when most have been retired
-                if (c->retire && l >= c->settle_from + c->chunk_first && generic_chunks > 2) most = std::max(4, most >> (generic_chunks - 2));
-            }
             // First launch of a pass that reads the input in place.  A layer that reads all N rows to compute
             // few classes is mostly loading: it pays only with several blocks of at least 8 images per SM, so
             // that one block's loads overlap another's arithmetic -- it takes the largest group that leaves
@@ -744,6 +748,19 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                 }
                 if (R0.mode == kResGeneric) {
                     if (ti == 32) ipt = maxc <= 256 ? 256 : maxc <= 512 ? 512 : 1024;      // inplace_kernel: threads per block
+                    // ... and so are the few images that are left when most have been retired: a second launch in smaller groups,
+                    // of which the device runs the one that suits the images it finds.  Images that stay unsaturated are never
+                    // retired, whatever the weights allow (1024 neurons, 60 layers of 32 entries, 20000 such images: 8346 us,
+                    // 18193 when late chunks always ran in small groups; the second launch costs 3 us where it is not needed).
+                    if (c->retire && l >= c->settle_from + c->chunk_first && generic_chunks > 2) {
+                        const int small = std::max(4, 32 >> std::min(generic_chunks - 2, 3));
+                        if (small < ti && fits(small, rows, 0)) {
+                            const int tb2 = (blob + 127) / 128 * 128;
+                            st.small_ti = small;
+                            st.small_table = c->stage_tables && fits(small, rows, tb2) ? tb2 : 0;
+                            st.small_images = small * c->sm_count;
+                        }
+                    }
                     // count_kernel pre-pass for tiles that are saturated already: uniform weight, 32 entries per class
                     // (its adder tree is built for 32), the two word buffers in shared memory
                     bool k32_all = k32 && R0.uniform;
@@ -832,6 +849,7 @@ enum { kFrontNone = 0, kFrontWords = 1, kFrontInPlace = 2, kFrontExpand = 3 };
 
 int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
     c->last_group = 0;
+    c->last_small = SmallGroups{};
     c->extra_launches = 0;
     c->streamed_launches = 0;
     c->retires = false;
@@ -944,9 +962,20 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
                     fprintf(stderr, "[spdnn] step %zu: pre-pass for saturated tiles (count form), layers %d..%d  %d threads per 32 images  %d words  smem %zu B\n",
                             step, l, l + st.count - 1, st.bits_threads, st.wwords, bsmem);
             }
+            a.live_from = st.small_ti ? st.small_images + 1 : 0;
+            a.live_to = 0x7fffffff;
             int rc = launch_resident(c, st.ti, st.ipt, a, grid, smem, R0.mode, R0.k == 32, R0.uniform);
             if (rc) return rc;
+            if (st.small_ti) {
+                ResArgs b = a;
+                b.live_from = 0; b.live_to = st.small_images; b.table_bytes = st.small_table;
+                rc = launch_resident(c, st.small_ti, 4, b, std::min((c->tiles_cap * 32 + st.small_ti - 1) / st.small_ti, c->sm_count),
+                                     resident_smem_bytes(st.small_ti, st.rows, st.small_table), R0.mode, R0.k == 32, R0.uniform);
+                if (rc) return rc;
+                c->extra_launches += 1;
+            }
             c->last_group = st.ti;
+            c->last_small = SmallGroups{(int)step, st.small_ti, st.small_images};
             char tables_txt[96];
             if (alt2 && st.tring) snprintf(tables_txt, sizeof tables_txt, "staged (%d layers per copy, %d copies in flight), %d word buffers", 1 << st.gshift, st.tring, st.wring);
             else if (alt2) snprintf(tables_txt, sizeof tables_txt, "global, %d word buffers", st.wring);
@@ -955,6 +984,8 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
                 fprintf(stderr, "[spdnn] step %zu: resident layers %d..%d  group %d images (%d per thread)  %s  rows %d (v_in %d, classes %d)  smem %zu B  tables %s%s\n",
                         step, l, l + st.count - 1, st.ti, st.ipt, R0.mode == kResAlt2 ? "ALT2" : "GENERIC", st.rows, R0.v_in,
                         R0.classes, smem, tables_txt, next_resident ? "  writes representatives only" : "");
+            if (c->print_schedule && st.small_ti)
+                fprintf(stderr, "[spdnn]         group %d images while at most %d are left  tables %s\n", st.small_ti, st.small_images, st.small_table ? "staged" : "global");
             if (c->print_schedule && st.dense) fprintf(stderr, "[spdnn]         reads the row-major input in place\n");
         } else {
             LayerDesc d;
@@ -1115,6 +1146,7 @@ int build_graph_kind(spdnn *c, int kind) {
     c->graph_steps[kind] = c->nsteps;
     c->graph_extra[kind] = c->extra_launches;
     c->graph_group[kind] = c->last_group;
+    c->graph_small[kind] = c->last_small;
     c->graph_expand_layer[kind] = c->expand_layer_of_plan;
     return SPDNN_OK;
 }
@@ -1618,6 +1650,7 @@ int spdnn_infer_async(spdnn_t *c) {
     c->nsteps = c->graph_steps[c->input_kind];
     c->extra_launches = c->graph_extra[c->input_kind];
     c->last_group = c->graph_group[c->input_kind];
+    c->last_small = c->graph_small[c->input_kind];
     c->final_expand_layer = c->graph_expand_layer[c->input_kind];
     c->final_needs_expand = c->final_expand_layer >= 0;
     CK(cudaGraphLaunch(c->graph_exec[c->input_kind], c->stream));
@@ -1666,7 +1699,7 @@ int spdnn_sync(spdnn_t *c, spdnn_stats_t *stats) {
         s.algorithmic_bytes = bytes;
         s.kernel_launches = c->nsteps + c->extra_launches + 1 + c->prep_launches;      // + finalize_kernel
         s.loop_launches = c->nsteps;
-        s.resident_group = c->last_group;
+        s.resident_group = c->last_small.ti && c->report.ctl[c->last_small.step].live <= c->last_small.images ? c->last_small.ti : c->last_group;
         c->stats = s;
         c->result_ready = true;
     }

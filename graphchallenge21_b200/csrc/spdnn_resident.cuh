@@ -113,6 +113,7 @@ struct ResArgs {
     // the launch runs only when *gate == gate_want (nullptr: always), see LayerArgs
     const int32_t *gate;
     int gate_want;
+    int live_from, live_to;   // GENERIC chunks: the launch runs only when the images on the work list are within these bounds
     Retire retire;
     int settle_from;          // from this layer of the chunk on to the end of the network every layer maps the all-clip vector onto itself
 };
@@ -401,6 +402,7 @@ resident_kernel(const ResArgs a) {
     const int sub = tid % LPC, grp = tid / LPC;
     const LoopCtl ctl = *a.ctl_in;
     const int live_in = ctl.live;
+    if (live_in < a.live_from || live_in > a.live_to) return;
     const int nblk = (live_in + TI - 1) / TI;
     const int buf_bytes = a.buf_rows * RS;
 
@@ -689,6 +691,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) inplace_kernel(const ResArgs a)
     const int sub = tid & 7, grp = tid >> 3;
     const LoopCtl ctl = *a.ctl_in;
     const int live_in = ctl.live;
+    if (live_in < a.live_from || live_in > a.live_to) return;
     for (int tile = blockIdx.x; tile < (live_in + 31) / 32; tile = next_group(a.work, &s_group)) {
         if (a.tile_done != nullptr && a.tile_done[tile] != 0) continue;
         const bool valid = tile * 32 + lane < live_in;

@@ -61,3 +61,30 @@ def test_binary_words_are_read_in_place(batch, bias, how, oracle):
             assert np.array_equal(g.layer_live(), want_l)
             assert np.array_equal(g.categories(), want_c)
             assert np.array_equal(g.activations(), want_a)
+
+
+@pytest.mark.parametrize("alternate", [False, True], ids=["one kind of layer", "a chunk per layer"])
+def test_images_that_stay_unsaturated_keep_their_groups(alternate, oracle):
+    """Every layer keeps the all-clip vector, but no image gets there: nothing is retired, and no chunk, however late, may
+    be run in the small groups meant for the few images left behind retired ones."""
+    n, L, k, b = 256, 60, 20, 2400
+    rng = np.random.default_rng(3)
+    layers = []
+    for l in range(L):
+        uniform = alternate and l % 2 == 1
+        rows = np.sort(np.argpartition(rng.random((n, n)), k, axis=1)[:, :k], axis=1).astype(np.int32)
+        if uniform:
+            rows[:, 16:] = -1
+        layers.append((rows, np.full((n, k), 1.0 / 16 if uniform else 1.002 / k, np.float32)))
+    y0 = (8 + 8 * rng.random((b, n))).astype(np.float32)
+    want_c, want_a, want_l = oracle.infer(y0, layers, 0.0)
+    with SpDNN(n, L, 0.0) as g:
+        for l, (rows, vals) in enumerate(layers):
+            g.set_layer_rows(l, rows, vals)
+        g.set_input_dense(y0)
+        res = g.infer()
+        assert np.array_equal(g.layer_live(), want_l) and len(want_c) == b
+        assert np.array_equal(g.activations(), want_a) and ((want_a > 0) & (want_a < 32)).all()
+        assert g.shortcuts()["retired_images"] == 0
+        assert res.loop_launches >= (L if alternate else 6)
+        assert res.resident_group >= 16
