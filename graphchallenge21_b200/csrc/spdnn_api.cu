@@ -16,6 +16,7 @@
 #include <memory>
 #include <new>
 #include <string>
+#include <tuple>
 #include <unordered_map>
 #include <vector>
 
@@ -75,6 +76,26 @@ struct DevRes {
 
 // The last resident step of a schedule runs in groups of ti when it finds at most `images` images (ti == 0: never).
 struct SmallGroups { int step = 0, ti = 0, images = 0; };
+
+struct Step;
+
+// A captured pass: one graph and what its launches are.
+struct Pass {
+    cudaGraphExec_t exec = nullptr;
+    int kind = 0;                      // of input (see spdnn::pass_of)
+    std::vector<Step> plan;            // a plan that equals it runs the same graph
+    int steps = 0, extra = 0, group = 0;
+    SmallGroups small;
+    int expand_layer = -1;             // the layer whose classes spdnn_get_activations must still expand to all member
+                                       // rows (-1: the tiles are complete)
+    Pass();
+    ~Pass();
+};
+
+// Batch sizes between which a plan may change, in images per SM (group_limit and the split first chunk of plan_steps say
+// why the lines lie there); batch class q lies above q of them.
+constexpr int kBatchEdges[] = {4, 8, 16, 32, 48, 128};
+constexpr int kBatchClasses = (int)(sizeof kBatchEdges / sizeof kBatchEdges[0]) + 1;
 
 }  // namespace
 
@@ -160,7 +181,6 @@ struct spdnn {
     int alt2_threads = 0;              // SPDNN_ALT2_THREADS=256|512: block size of ALT2 chunks with 4 images per thread (0: by shared memory)
     int bits_threads = 0;              // SPDNN_BITS_THREADS: threads per block of the pre-pass (0: by the classes)
     int extra_launches = 0;            // pre-pass launches of the captured schedule
-    int graph_extra[2] = {0, 0};
     int32_t *ids[2] = {nullptr, nullptr};
     unsigned int *counter = nullptr;   // [0] blocks finished, [1] next work item, [2] images retired by a launch, [3] layers skipped in this pass
     int32_t *status = nullptr;
@@ -171,17 +191,16 @@ struct spdnn {
 
     int batch = 0, first_id = 0;
     bool input_ready = false, result_ready = false, in_flight = false, prep_timed = false;
-    // One captured pass per kind of input: [0] the input is in tiles (y[0]); [1] the first launch reads the
-    // caller's row-major matrix in place (only when that launch is a resident chunk; else null).
-    cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
-    int graph_steps[2] = {0, 0}, graph_group[2] = {0, 0};
-    SmallGroups graph_small[2];
+    // The captured pass for each kind of input and class of batch, built when a batch first needs it: [0] the input is in
+    // tiles (y[0]); [1] the first launch reads the caller's row-major matrix in place (only when that launch is a resident
+    // chunk; else null).  Classes with equal plans share a pass.
+    Pass *pass_of[2][kBatchClasses] = {};
+    bool no_pass_of[2][kBatchClasses] = {};                 // planned: there is none for this kind
+    std::vector<std::unique_ptr<Pass>> passes;
     bool graph_dirty = true;
     bool alt2_small_blocks = true;     // SPDNN_ALT2_SMALL_BLOCKS=0: 256-thread blocks also for layers of <= 64 classes
     bool lazy_expand = true;           // SPDNN_LAZY_EXPAND=0: the last launch of a pass writes all member rows itself
     int expand_layer_of_plan = -1;     // set by enqueue_layers
-    int graph_expand_layer[2] = {-1, -1};   // per captured pass: the layer whose classes spdnn_get_activations must
-                                            // still expand to all member rows (-1: the tiles are complete)
     bool final_needs_expand = false;   // ... pending for the pass that ran last
     int final_expand_layer = -1;
     bool dense_direct = false;         // SPDNN_DENSE_DIRECT=1: let the first launch read a dense input in place where
@@ -582,10 +601,25 @@ struct Step {
     unsigned char *cache = nullptr;
     unsigned short *rec_of = nullptr;
     int cache_records = 0;
+    int most_images = 0x7fffffff;      // GENERIC chunk: the largest batch of the plan's class, which the blocks are counted for
     // GENERIC chunk: groups of small_ti images instead when at most small_images are on the work list (0: no such launch)
     int small_ti = 0, small_table = 0, small_images = 0;
     int period = 0, period_from = 0;      // ALT2 chunk: its tables repeat with this period from this layer of the chunk on (0: no)
+
+    // The shape of the launch (stream, cache and rec_of are made from it when the pass is captured).
+    bool same_shape(const Step &o) const {
+        auto shape = [](const Step &x) {
+            return std::make_tuple(x.first, x.count, x.ti, x.ipt, x.rows, x.table, x.stride, x.gshift, x.tring, x.wring, x.rows_w, x.max_classes, x.dense,
+                                   x.bits_threads, x.bits_gshift, x.bits_tring, x.wwords, x.small_ti, x.small_table, x.small_images, x.period, x.period_from, x.most_images);
+        };
+        return shape(*this) == shape(o);
+    }
 };
+
+Pass::Pass() = default;
+Pass::~Pass() {
+    if (exec) cudaGraphExecDestroy(exec);
+}
 
 // Period of an ALT2 chunk's tables: the smallest P such that the chunk ends in at least two periods of layers whose
 // tables (matrix and value ids) repeat with P, and the first layer of that part.
@@ -602,11 +636,43 @@ void find_period(spdnn *c, Step &st) {
     }
 }
 
+int batch_class_of(const spdnn *c, int images) {
+    int q = 0;
+    while (q < kBatchClasses - 1 && images > kBatchEdges[q] * c->sm_count) ++q;
+    return q;
+}
+
+// Whether a batch class lies above `edge` (one of kBatchEdges).
+bool above(int batch_class, int edge) {
+    for (int q = 0; q < batch_class; ++q)
+        if (kBatchEdges[q] == edge) return true;
+    return false;
+}
+
+// Most images per block of a GENERIC chunk.  A block's time grows with its images, but less than in proportion (one
+// block per SM, 16 layers of 32 general weights at 1024 neurons: 210, 270, 360 and 452 us for 4, 8, 16 and 32 images), and
+// blocks that share an SM take almost as long as one after the other (700 images in groups of 4: 382 us).  So a group is as
+// small as one block per SM allows, up to 16; 32 (inplace_kernel) pays with at least 12 entries, which its two barriers
+// and its table copies per layer cost as much as, and
+//   more than 256 classes    as soon as 16 images would need a second block per SM (us for 16 and 32: 1024 classes, 32
+//                            entries, 2800 images 700, 452, 20000 images 3118, 2201, but 4 entries 792, 833; 512
+//                            classes, 20 entries, 2800 images 214, 196, 20000 images 907, 735);
+//   up to 256 classes        its blocks have 256 threads: with the fourth block of 16 (20 entries, 5500 images 186, 190,
+//                            9400 images 249, 194).
+// Uniform layers of many classes and entries bear two blocks of 4 per SM (random networks of 1024 neurons, 40 layers, 1100
+// images: 284 us, in groups of 8 297).
+int group_limit(const DevRes &R, int batch_class) {
+    if (!above(batch_class, 4)) return 4;
+    if (!above(batch_class, 8)) return R.classes > 512 && R.uniform && R.k >= 24 ? 4 : 8;
+    return R.k >= 12 && above(batch_class, R.classes > 256 ? 16 : 48) ? 32 : 16;
+}
+
 // The launches of one pass, front to back.
 // dense_first: the pass starts from the caller's row-major input; its first launch is then a resident
 // chunk wherever one fits (Step::dense), because loading the rows into shared memory also does the change
 // of layout.
-std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
+// batch_class: the class of the batch the plan is for; the plan may depend on nothing else that changes between passes.
+std::vector<Step> plan_steps(spdnn *c, bool dense_first, int batch_class) {
     std::vector<Step> plan;
     int l = 0, chunk = c->chunk_list.empty() ? c->chunk_first : c->chunk_list[0];
     int resident_chunks = 0;       // resident chunks planned so far
@@ -634,11 +700,7 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
             static const int kGeneric[][2] = {{32, 4}, {16, 4}, {8, 4}, {4, 4}};
             const int (*cand)[2] = R0.mode == kResAlt2 ? kAlt2 : kGeneric;
             const int ncand = R0.mode == kResAlt2 ? 5 : 4;
-            // GENERIC groups: as many images as still give every SM a block; a block's time grows with its images, so a
-            // small batch is faster in smaller groups on more SMs
-            int most = 32;
-            if (R0.mode == kResGeneric)
-                while (most > 4 && c->tiles_cap * (32 / most) < c->sm_count) most /= 2;
+            const int most = R0.mode == kResGeneric ? group_limit(R0, batch_class) : 32;
             // First launch of a pass that reads the input in place.  A layer that reads all N rows to compute
             // few classes is mostly loading: it pays only with several blocks of at least 8 images per SM, so
             // that one block's loads overlap another's arithmetic -- it takes the largest group that leaves
@@ -662,11 +724,11 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                 // extend while the layers are of one kernel variant and the group still fits
                 int f = 1, blob = R0.blob_bytes, maxc = R0.classes;
                 if (R0.mode == kResAlt2 && alt2_chunks == 0 && chunk == 8 && own_lengths) {
-                    // Blocks that fill an SM and many of them: two thirds of the images die within the first eight layers, and the
+                    // Blocks that fill an SM and at least eight of them for each: two thirds of the images die within the first eight layers, and the
                     // second four without the dead cost less than the launch between (16384 neurons, layer loop: 60000 images
                     // 1703 -> 1617 us, 6000 images 298 -> 317).
                     split = ti == 16 && resident_smem_bytes(ti, rows, 0) * 2 + 4096 > (size_t)c->smem_optin &&
-                            (long long)c->tiles_cap * 32 >= 16LL * 8 * c->sm_count;
+                            above(batch_class, 128);
                     if (split) chunk = 4;
                 }
                 while (f < chunk && l + f < c->layers && c->res[l + f]) {
@@ -747,13 +809,14 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first) {
                     }
                 }
                 if (R0.mode == kResGeneric) {
+                    st.most_images = batch_class < kBatchClasses - 1 ? kBatchEdges[batch_class] * c->sm_count : 0x7fffffff;
                     if (ti == 32) ipt = maxc <= 256 ? 256 : maxc <= 512 ? 512 : 1024;      // inplace_kernel: threads per block
                     // ... and so are the few images that are left when most have been retired: a second launch in smaller groups,
                     // of which the device runs the one that suits the images it finds.  Images that stay unsaturated are never
                     // retired, whatever the weights allow (1024 neurons, 60 layers of 32 entries, 20000 such images: 8346 us,
                     // 18193 when late chunks always ran in small groups; the second launch costs 3 us where it is not needed).
                     if (c->retire && l >= c->settle_from + c->chunk_first && generic_chunks > 2) {
-                        const int small = std::max(4, 32 >> std::min(generic_chunks - 2, 3));
+                        const int small = ti == 32 && generic_chunks == 3 ? 16 : 4;
                         if (small < ti && fits(small, rows, 0)) {
                             const int tb2 = (blob + 127) / 128 * 128;
                             st.small_ti = small;
@@ -907,7 +970,7 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
             a.n = c->n; a.bias = c->bias; a.clip = c->clip;
             a.reps_only = (next_resident || lazy_last) ? 1 : 0;
             a.exact_ok = (l > 0 && c->clip <= 1024.0f && c->exact_shortcut) ? 1 : 0;
-            const int grid = std::max(1, (c->tiles_cap * 32 + st.ti - 1) / st.ti);
+            const int grid = std::max(1, (std::min(c->tiles_cap * 32, st.most_images) + st.ti - 1) / st.ti);
             const bool alt2 = (R0.mode == kResAlt2);
             const size_t smem = alt2 ? alt2_smem_bytes(st.ti, st.rows, st.stride, st.gshift, st.tring)
                               : st.ti == 32 ? inplace_smem_bytes(st.rows, st.ipt / 32, st.table) : resident_smem_bytes(st.ti, st.rows, st.table);
@@ -969,7 +1032,7 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
             if (st.small_ti) {
                 ResArgs b = a;
                 b.live_from = 0; b.live_to = st.small_images; b.table_bytes = st.small_table;
-                rc = launch_resident(c, st.small_ti, 4, b, std::min((c->tiles_cap * 32 + st.small_ti - 1) / st.small_ti, c->sm_count),
+                rc = launch_resident(c, st.small_ti, 4, b, (std::min(c->tiles_cap * 32, st.small_images) + st.small_ti - 1) / st.small_ti,
                                      resident_smem_bytes(st.small_ti, st.rows, st.small_table), R0.mode, R0.k == 32, R0.uniform);
                 if (rc) return rc;
                 c->extra_launches += 1;
@@ -1087,10 +1150,21 @@ int enqueue_layers(spdnn *c, const std::vector<Step> &plan, bool gated) {
     return SPDNN_OK;
 }
 
-// Captures the launches of one pass for one kind of input (0: tiles, 1: row-major read in place).
-int build_graph_kind(spdnn *c, int kind) {
-    std::vector<Step> plan = plan_steps(c, kind == 1);
-    if (kind == 1 && !(plan[0].ti && plan[0].dense)) return SPDNN_OK;      // no resident first launch: kind 0 serves
+// Captures the launches of one pass for one kind of input (0: tiles, 1: row-major read in place) and class of batch.
+int build_pass(spdnn *c, int kind, int batch_class) {
+    std::vector<Step> plan = plan_steps(c, kind == 1, batch_class);
+    if (kind == 1 && !(plan[0].ti && plan[0].dense)) {                     // no resident first launch: kind 0 serves
+        c->no_pass_of[kind][batch_class] = true;
+        return SPDNN_OK;
+    }
+    for (const auto &p : c->passes) {
+        bool same = p->kind == kind && p->plan.size() == plan.size();
+        for (size_t q = 0; same && q < plan.size(); ++q) same = p->plan[q].same_shape(plan[q]);
+        if (same) {
+            c->pass_of[kind][batch_class] = p.get();
+            return SPDNN_OK;
+        }
+    }
     // outside the capture: the packed table stream of every ALT2 chunk
     for (Step &st : plan) {
         if (!st.ti || c->res[st.first]->mode != kResAlt2) continue;
@@ -1140,20 +1214,34 @@ int build_graph_kind(spdnn *c, int kind) {
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
     if (e != cudaSuccess) return fail(c, SPDNN_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&c->graph_exec[kind], g, 0);
+    auto pass = std::make_unique<Pass>();
+    e = cudaGraphInstantiate(&pass->exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(c, SPDNN_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e));
-    c->graph_steps[kind] = c->nsteps;
-    c->graph_extra[kind] = c->extra_launches;
-    c->graph_group[kind] = c->last_group;
-    c->graph_small[kind] = c->last_small;
-    c->graph_expand_layer[kind] = c->expand_layer_of_plan;
+    pass->kind = kind;
+    pass->steps = c->nsteps;
+    pass->extra = c->extra_launches;
+    pass->group = c->last_group;
+    pass->small = c->last_small;
+    pass->expand_layer = c->expand_layer_of_plan;
+    pass->plan.swap(plan);
+    c->pass_of[kind][batch_class] = pass.get();
+    c->passes.push_back(std::move(pass));
     return SPDNN_OK;
 }
 
-int build_graph(spdnn *c) {
+void drop_passes(spdnn *c) {
     for (int kind = 0; kind < 2; ++kind)
-        if (c->graph_exec[kind]) { cudaGraphExecDestroy(c->graph_exec[kind]); c->graph_exec[kind] = nullptr; }
+        for (int q = 0; q < kBatchClasses; ++q) {
+            c->pass_of[kind][q] = nullptr;
+            c->no_pass_of[kind][q] = false;
+        }
+    c->passes.clear();
+}
+
+// Everything the passes of a network have in common.
+int build_graph(spdnn *c) {
+    drop_passes(c);
     for (unsigned char *p : c->streams) cudaFree(p);
     c->streams.clear();
     int rc = prepare_resident(c);
@@ -1174,22 +1262,31 @@ int build_graph(spdnn *c) {
             c->wslot_bytes = need;
         }
     }
-    rc = build_graph_kind(c, 0);
-    if (rc) return rc;
-    if (c->dense_direct && c->resident) {
-        rc = build_graph_kind(c, 1);
-        if (rc) return rc;
-    }
     c->graph_dirty = false;
     return SPDNN_OK;
 }
 
-// Builds the graphs if every layer has been set; returns false (without an error) when it cannot yet.
-bool graphs_ready(spdnn *c) {
-    if (!c->graph_dirty) return true;
+// *pass: what the current batch runs for this kind of input, built if it is not there yet (null: the kind cannot serve).
+int find_pass(spdnn *c, int kind, Pass **pass) {
+    *pass = nullptr;
+    if (c->graph_dirty) {
+        if (int rc = build_graph(c)) return rc;
+    }
+    if (kind == 1 && !(c->dense_direct && c->resident)) return SPDNN_OK;
+    const int q = batch_class_of(c, c->batch);
+    if (!c->pass_of[kind][q] && !c->no_pass_of[kind][q]) {
+        if (int rc = build_pass(c, kind, q)) return rc;
+    }
+    *pass = c->pass_of[kind][q];
+    return SPDNN_OK;
+}
+
+// Whether the pass to come can read a row-major input in place; false (without an error) when that cannot be said yet.
+bool reads_dense_in_place(spdnn *c) {
     for (int l = 0; l < c->layers; ++l)
         if (!c->layer[l]) return false;
-    return build_graph(c) == SPDNN_OK;
+    Pass *pass = nullptr;
+    return find_pass(c, 1, &pass) == SPDNN_OK && pass != nullptr;
 }
 
 struct DeviceGuard {
@@ -1308,8 +1405,7 @@ void spdnn_destroy(spdnn_t *c) {
     if (!c) return;
     DeviceGuard guard(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (int kind = 0; kind < 2; ++kind)
-        if (c->graph_exec[kind]) cudaGraphExecDestroy(c->graph_exec[kind]);
+    drop_passes(c);
     cudaFree(c->dense_cell); cudaFree(c->first_cell);
     free_buffers(c);
     cudaFree(c->ctl); cudaFree(c->counter); cudaFree(c->status); cudaFree(c->stage);
@@ -1478,7 +1574,7 @@ int spdnn_set_input_dense_device(spdnn_t *c, const float *y0_dev, int batch, int
     DeviceGuard guard(c->device);
     int rc = begin_input(c, batch, first_global_id);
     if (rc) return rc;
-    if (batch > 0 && c->dense_direct && graphs_ready(c) && c->graph_exec[1]) {
+    if (batch > 0 && c->dense_direct && reads_dense_in_place(c)) {
         c->dense_src = y0_dev;       // read in place by the first launch of the pass
         c->input_kind = 1;
         return end_input(c);
@@ -1496,7 +1592,7 @@ int spdnn_set_input_dense(spdnn_t *c, const float *y0, int batch, int first_glob
     int rc = begin_input(c, batch, first_global_id);
     if (rc) return rc;
     const size_t row_bytes = sizeof(float) * (size_t)c->n;
-    if (batch > 0 && c->dense_direct && (size_t)batch * row_bytes <= ((size_t)1 << 30) && graphs_ready(c) && c->graph_exec[1]) {
+    if (batch > 0 && c->dense_direct && (size_t)batch * row_bytes <= ((size_t)1 << 30) && reads_dense_in_place(c)) {
         // one copy into the staging buffer, which the first launch of the pass reads in place
         rc = ensure_stage(c, (size_t)batch * row_bytes);
         if (rc) return rc;
@@ -1640,20 +1736,17 @@ int spdnn_infer_async(spdnn_t *c) {
     for (int l = 0; l < c->layers; ++l)
         if (!c->layer[l]) return fail(c, SPDNN_ERR_STATE, "layer %d was never set", l);
     DeviceGuard guard(c->device);
-    if (c->graph_dirty) {
-        int rc = build_graph(c);
-        if (rc) return rc;
-    }
+    Pass *pass = nullptr;
+    if (int rc = find_pass(c, c->input_kind, &pass)) return rc;
+    if (!pass) return fail(c, SPDNN_ERR_STATE, "the network changed after the input was set: set the input again");
     CK(cudaEventRecord(c->ev_inf0, c->stream));
-    if (c->input_kind == 1 && !c->graph_exec[1])
-        return fail(c, SPDNN_ERR_STATE, "the network changed after the input was set: set the input again");
-    c->nsteps = c->graph_steps[c->input_kind];
-    c->extra_launches = c->graph_extra[c->input_kind];
-    c->last_group = c->graph_group[c->input_kind];
-    c->last_small = c->graph_small[c->input_kind];
-    c->final_expand_layer = c->graph_expand_layer[c->input_kind];
+    c->nsteps = pass->steps;
+    c->extra_launches = pass->extra;
+    c->last_group = pass->group;
+    c->last_small = pass->small;
+    c->final_expand_layer = pass->expand_layer;
     c->final_needs_expand = c->final_expand_layer >= 0;
-    CK(cudaGraphLaunch(c->graph_exec[c->input_kind], c->stream));
+    CK(cudaGraphLaunch(pass->exec, c->stream));
     CK(cudaEventRecord(c->ev_inf1, c->stream));
     c->input_ready = false;
     c->in_flight = true;

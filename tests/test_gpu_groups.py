@@ -1,5 +1,6 @@
-"""GPU tests of the group sizes of GENERIC chunks: the batch decides how many images a block holds (32 with one buffer and
-the outputs in registers, 16, 8 or 4 with two), every size against the oracle, bit for bit."""
+"""GPU tests of the group sizes of GENERIC chunks: the batch, the classes and the entries of a layer decide how many images a
+block holds (32 with one buffer and the outputs in registers, 16, 8 or 4 with two), every size against the oracle, bit for
+bit."""
 import numpy as np
 import pytest
 
@@ -22,7 +23,7 @@ def network(n, L, k, seed):
     return out
 
 
-@pytest.mark.parametrize("batch", [4737, 2400, 1190, 70])           # 32, 16, 8 and 4 images a block on 148 SMs
+@pytest.mark.parametrize("batch", [4737, 2400, 1190, 70])
 @pytest.mark.parametrize("n,k,L", [(96, 20, 11), (256, 37, 9), (512, 32, 9), (700, 9, 4), (1024, 32, 10)])
 def test_general_weights(n, k, L, batch, oracle):
     layers = network(n, L, k, n + k)
@@ -88,3 +89,87 @@ def test_images_that_stay_unsaturated_keep_their_groups(alternate, oracle):
         assert g.shortcuts()["retired_images"] == 0
         assert res.loop_launches >= (L if alternate else 6)
         assert res.resident_group >= 16
+
+
+def sm_count():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("n,k,L,uniform,per_sm,above,group",
+                         [(96, 20, 5, False, 4, 0, 4), (96, 20, 5, False, 8, 1, 16), (96, 20, 5, False, 48, 1, 32),
+                          (256, 37, 4, False, 4, 1, 8), (256, 37, 4, False, 48, 0, 16), (256, 37, 4, False, 48, 1, 32), (256, 32, 4, True, 8, 0, 8),
+                          (512, 32, 4, False, 4, 0, 4), (512, 32, 4, False, 8, 0, 8), (512, 32, 4, False, 16, 0, 16), (512, 32, 4, False, 16, 1, 32),
+                          (512, 32, 4, False, 32, 1, 32), (512, 32, 4, True, 8, 0, 8), (700, 9, 4, False, 4, 1, 8), (700, 9, 4, False, 16, 0, 16),
+                          (700, 9, 4, False, 16, 1, 32), (700, 8, 4, False, 48, 1, 16), (1024, 32, 10, False, 4, 0, 4), (1024, 32, 10, False, 4, 1, 8),
+                          (1024, 32, 10, False, 8, 1, 16), (1024, 32, 10, False, 16, 0, 16), (1024, 32, 10, False, 16, 1, 32),
+                          (1024, 32, 4, True, 4, 0, 4), (1024, 32, 4, True, 8, 0, 4), (1024, 32, 4, True, 8, 1, 16), (1024, 20, 4, True, 8, 0, 8),
+                          (1024, 32, 4, True, 16, 1, 32)])
+def test_every_group_size_on_either_side_of_its_limits(n, k, L, uniform, per_sm, above, group, oracle):
+    layers = network(n, L, k, n + k)
+    if uniform:
+        layers = [(rows, None) for rows, _ in layers]
+    batch = per_sm * sm_count() + above              # the last batch of a class, or the first of the next
+    y0 = mixed_density_images(n, batch)
+    bias = -0.3 if uniform else -0.25
+    want_c, want_a, want_l = oracle.infer(y0, layers, bias)
+    with SpDNN(n, L, bias) as g:
+        for l, (rows, vals) in enumerate(layers):
+            g.set_layer_rows(l, rows, vals)
+        g.set_input_dense(y0)
+        res = g.infer()
+        assert res.resident_group == group
+        assert np.array_equal(g.layer_live(), want_l)
+        assert np.array_equal(g.categories(), want_c)
+        assert np.array_equal(g.activations(), want_a)
+
+
+@pytest.mark.parametrize("n,k,big,small", [(256, 37, 6000, 64), (512, 20, 6000, 700), (1024, 32, 6000, 64), (1024, 4, 5000, 900)])
+def test_a_small_batch_runs_alike_whatever_the_context_has_served(n, k, big, small, oracle):
+    """The plan follows the batch, not the buffers: sizes in turn through one context, each as in a context of its own."""
+    L = 5
+    layers = network(n, L, k, n + k)
+    y0 = mixed_density_images(n, big)
+
+    def context():
+        g = SpDNN(n, L, -0.25)
+        for l, (rows, vals) in enumerate(layers):
+            g.set_layer_rows(l, rows, vals)
+        return g
+
+    with context() as used:
+        for b in (big, small, big, 1, small):
+            y = y0[:b] * np.float32(0.9 if b == small else 1.0)
+            want_c, want_a, want_l = oracle.infer(y, layers, -0.25)
+            used.set_input_dense(y)
+            res = used.infer()
+            with context() as fresh:
+                fresh.set_input_dense(y)
+                own = fresh.infer()
+            assert (res.resident_group, res.loop_launches) == (own.resident_group, own.loop_launches)
+            assert np.array_equal(used.layer_live(), want_l)
+            assert np.array_equal(used.categories(), want_c)
+            assert np.array_equal(used.activations(), want_a)
+
+
+def test_only_full_batches_split_their_first_chunk(oracle):
+    n, L = 16384, 24
+    net = SyntheticNetwork(n, L, "radix16")
+    big = 128 * sm_count() + 1
+    rng = np.random.default_rng(1)
+    bits = rng.integers(0, 256, (big, n // 8), dtype=np.uint8)
+    y0 = mixed_density_images(n, 40)
+    want_c, want_a, want_l = oracle.infer(y0, [(net.layer_rows(l), None) for l in range(L)], float(net.bias))
+    with SpDNN(n, L, float(net.bias)) as g:
+        g.set_network(net)
+        g.set_input_dense(y0)
+        fresh = g.infer().loop_launches
+        g.set_input_bits(bits)
+        assert g.infer().loop_launches == fresh + 1
+        g.set_input_bits(bits[:-1])
+        assert g.infer().loop_launches == fresh
+        g.set_input_dense(y0)
+        assert g.infer().loop_launches == fresh
+        assert np.array_equal(g.layer_live(), want_l)
+        assert np.array_equal(g.categories(), want_c)
+        assert np.array_equal(g.activations(), want_a)
