@@ -868,13 +868,15 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first, int batch_class) {
                 } else {
                     chunk = std::min(chunk * (alt2 ? c->chunk_growth : c->chunk_growth_generic), c->chunk_max);
                     // Images without structure saturate one by one soon after the first chunk, at clip everywhere, and leave the
-                    // list at the end of a chunk: chunks of 2, 2, 4, 8, ... layers follow the first one (59 % of the survivors are gone at
-                    // layer 8 of such a network of 1024 neurons, 89 % at 10, 96 % at 12; with 16 layers after the first 8 the float form
-                    // ran them all for everyone: 3866 us for 60000 images, in the short chunks 640).
-                    if (!alt2 && c->retire && !c->chunk_growth_set && l + st.count >= c->settle_from) {
-                        if (generic_chunks == 0) chunk = std::min(chunk, 2);
-                        else if (generic_chunks == 1) chunk = std::min(chunk, 2);
-                    }
+                    // list at the end of a chunk: for large batches chunks of 2, 2, 4, 8, ... layers follow the first one (random
+                    // network of 1024 neurons, 120 layers: of 33190 survivors of 60000 images 13785 are not all clip after layer 7,
+                    // 3470 after layer 9, 975 after layer 11; 3265 us against 3509 with 8, 16, 32, ...).  Below 48 images per SM
+                    // blocks whose images have all arrived end early enough by themselves, and the launches between cost more
+                    // (64 images 245 us against 211, 6000 images 739 against 712); so they do where layers have few entries (4
+                    // entries, 20000 images that stay unsaturated, 60 layers: 3119 against 2902).
+                    if (!alt2 && c->retire && !c->chunk_growth_set && l + st.count >= c->settle_from && generic_chunks < 2 &&
+                        above(batch_class, 48) && c->res[l]->k >= 12)
+                        chunk = std::min(chunk, 2);
                 }
                 // Where the tables repeat, alt2_kernel's own bit form ends a tile one period after it saturates
                 // (ResArgs::period): from the third ALT2 chunk on one launch takes the rest of the network, provided that

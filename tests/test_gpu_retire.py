@@ -52,3 +52,20 @@ def test_retired_images_are_survivors(kind, n, b, L, env, monkeypatch, oracle):
         assert np.array_equal(live, wl)
         assert np.array_equal(cats, wc) and survivors == len(wc)
         assert np.array_equal(act, wa)
+
+
+def test_large_batches_retire_in_short_chunks(oracle):
+    import torch
+    n, L, b = 1024, 26, 48 * torch.cuda.get_device_properties(0).multi_processor_count + 37
+    net = SyntheticNetwork(n, L, "random")
+    y0 = mixed_density_images(n, b)
+    want_c, want_a, want_l = oracle.infer(y0, [(r, None) for r in rows_of(net)], float(net.bias), first_image=11)
+    with SpDNN(n, L, float(net.bias)) as g:
+        g.set_network(net)
+        g.set_input_dense(y0, 11)
+        res = g.infer()
+        assert res.loop_launches == 6                            # 8, 2, 2, 4, 8, 2 layers
+        assert g.shortcuts()["retired_images"] > 0.4 * b
+        assert np.array_equal(g.layer_live(), want_l)
+        assert np.array_equal(g.categories(), want_c)
+        assert np.array_equal(g.activations(), want_a)
