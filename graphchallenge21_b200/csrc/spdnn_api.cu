@@ -688,6 +688,10 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first, int batch_class) {
             const DevRes &R0 = *c->res[l];
             const bool k32 = (R0.k == 32);
             int kmax = R0.k;               // most entries per class in the chunk
+            if (short_chunk > 0 && R0.mode != kResAlt2) {      // (the rest of the network at once is for ALT2 layers, see below)
+                chunk = short_chunk;
+                short_chunk = 0;
+            }
             auto fits = [&](int t_i, int r, int table) {
                 const size_t need = R0.mode == kResGeneric && t_i == 32 ? inplace_smem_bytes(r, 32, inplace_table_bytes(kmax, R0.uniform))
                                                                        : resident_smem_bytes(t_i, r, table);
