@@ -791,11 +791,11 @@ std::vector<Step> plan_steps(spdnn *c, bool dense_first, int batch_class) {
                     }
                     // Pre-pass for tiles that are saturated already (bits_kernel): layers of more than one pass of 64
                     // classes, where the float buffers leave this kernel's own bit form few images per block.  Not
-                    // before the first two chunks of a pass: the challenge networks saturate around layer 30, and a
-                    // tile that is not saturated costs the pre-pass a read of all its rows for nothing.
+                    // before the first two chunks of a pass (a split first chunk counts once): the challenge networks saturate around
+                    // layer 30, and a tile that is not saturated costs the pre-pass a read of all its rows for nothing.
                     const int rows_max = std::max(rows, maxc);
                     if (c->bits_prepass && c->bit_form && c->clip > 0.0f && (maxc > 64 || c->bits_small) && rows_max <= 16383 &&
-                        ((alt2_chunks > 1 && l > 12) || c->bits_first_chunk)) {
+                        (alt2_chunks - (split ? 1 : 0) > 1 || c->bits_first_chunk)) {
                         st.wwords = (rows_max + 63) / 64 * 64;
                         const int passes = (maxc + 63) / 64;
                         int nt = c->bits_threads > 0 ? c->bits_threads : 32 * ((passes + 1) / 2);

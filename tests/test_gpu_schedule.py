@@ -44,3 +44,18 @@ def test_only_alt2_layers_take_the_rest_of_the_network_at_once(capfd, monkeypatc
     lines = schedule(capfd, monkeypatch, oracle, n, layers, float(a.bias), y0)
     assert chunks(lines, "ALT2") == [(1, 8), (9, 19)]
     assert chunks(lines, "GENERIC") == [(20, 147), (148, 239)]
+
+
+@pytest.mark.parametrize("lengths,first", [("3,3,32", 7), ("1,1,1,60", 3), ("8,32", 41), ("20,20", None)])
+def test_the_third_alt2_chunk_gets_the_pre_pass(lengths, first, capfd, monkeypatch, oracle):
+    """... however short the first two are."""
+    monkeypatch.setenv("SPDNN_CHUNKS", lengths)
+    n, L = 4096, 60 if first else 40
+    net = SyntheticNetwork(n, L, "radix16")
+    y0 = synthetic_images(n, 70)
+    y0[:32] *= np.float32(32.0)                                  # a tile that is saturated from the start
+    lines = schedule(capfd, monkeypatch, oracle, n, [(net.layer_rows(l), None) for l in range(L)], float(net.bias), y0)
+    found = [re.search(r"pre-pass for saturated tiles, layers (\d+)\.\.", line) for line in lines]
+    starts = [int(m[1]) for m in found if m]
+    assert starts[:1] == ([first] if first else [])
+    assert starts == [c[0] for c in chunks(lines, "ALT2")][2:]
