@@ -152,6 +152,7 @@ struct spdnn {
     int nsteps = 0;                    // launches of the last captured schedule
     std::vector<int32_t> host_live;
     HostReport report{};               // page-locked host memory the last launch of a pass writes its results to (ids: sized with the batch)
+    unsigned char *per_tile = nullptr;    // the block that holds slot, mask and the other small arrays sized with the batch
     int32_t *slot = nullptr;
     uint32_t *mask = nullptr;
     unsigned char *tile_done = nullptr;   // [tiles] verdict of the bits_kernel pre-pass of an ALT2 chunk
@@ -235,16 +236,14 @@ int fail(spdnn *c, int code, const char *fmt, ...) {
                         __FILE__, __LINE__);                                                          \
     } while (0)
 
-// has_floats lies behind in_flag in one allocation, so that one memset resets both
+// has_floats lies behind in_flag, so that one memset resets both
 constexpr size_t kMarksOffset = 16;
 
 int free_buffers(spdnn *c) {
-    cudaFree(c->y[0]); cudaFree(c->y[1]); cudaFree(c->slot); cudaFree(c->mask); cudaFree(c->tile_done);
-    cudaFree(c->ids[0]); cudaFree(c->ids[1]); cudaFree(c->xw); cudaFree(c->in_flag);
-    cudaFree(c->open_mask); cudaFree(c->settled); cudaFree(c->working); cudaFree(c->work_of);
-    c->open_mask = c->settled = c->working = nullptr; c->work_of = nullptr;
-    c->y[0] = c->y[1] = nullptr; c->slot = nullptr; c->mask = nullptr; c->ids[0] = c->ids[1] = nullptr;
-    c->tile_done = nullptr; c->xw = nullptr; c->has_floats = nullptr; c->in_flag = nullptr;
+    cudaFree(c->y[0]); cudaFree(c->y[1]); cudaFree(c->xw); cudaFree(c->per_tile);
+    c->y[0] = c->y[1] = nullptr; c->xw = nullptr; c->per_tile = nullptr;
+    c->open_mask = c->settled = c->working = c->mask = nullptr; c->work_of = c->slot = nullptr; c->ids[0] = c->ids[1] = nullptr;
+    c->tile_done = nullptr; c->has_floats = nullptr; c->in_flag = nullptr;
     cudaFreeHost(c->report.ctl);
     c->report = HostReport{};
     c->result_ready = c->input_ready = false;      // (their memory is gone)
@@ -262,7 +261,6 @@ int ensure_capacity(spdnn *c, int batch) {
     for (int i = 0; i < 2; ++i) {
         CK(cudaMalloc(&c->y[i], ybytes));
         CK(cudaMemsetAsync(c->y[i], 0, ybytes, c->stream));      // incl. the permanent zero row of every tile
-        CK(cudaMalloc(&c->ids[i], sizeof(int32_t) * (size_t)tiles * 32));
     }
     {
         // one block: the records per launch boundary, the deaths per layer, the status, the layers skipped, the image numbers
@@ -275,21 +273,32 @@ int ensure_capacity(spdnn *c, int batch) {
         c->report.skipped = reinterpret_cast<uint32_t *>(c->report.status + 1);
         c->report.ids = c->report.status + 2;
     }
-    CK(cudaMalloc(&c->slot, sizeof(int32_t) * (size_t)tiles * 32));
-    CK(cudaMalloc(&c->mask, sizeof(uint32_t) * (size_t)tiles));
-    CK(cudaMemsetAsync(c->mask, 0, sizeof(uint32_t) * (size_t)tiles, c->stream));
-    CK(cudaMalloc(&c->open_mask, sizeof(uint32_t) * (size_t)tiles));
-    CK(cudaMemsetAsync(c->open_mask, 0, sizeof(uint32_t) * (size_t)tiles, c->stream));
-    CK(cudaMalloc(&c->settled, sizeof(uint32_t) * (size_t)tiles));
-    CK(cudaMalloc(&c->working, sizeof(uint32_t) * (size_t)tiles));
-    CK(cudaMalloc(&c->work_of, sizeof(int32_t) * (size_t)tiles * 32));
-    CK(cudaMalloc(&c->tile_done, (size_t)tiles));
-    CK(cudaMemsetAsync(c->tile_done, 0, (size_t)tiles, c->stream));
+    {
+        // one block too (an allocation of its own for each cost a new context up to 0.4 ms a piece): everything that is small
+        // and sized with the batch, zero at first (the masks and marks are zero between passes)
+        size_t bytes = 0;
+        auto place = [&](size_t b) { const size_t at = bytes; bytes = (bytes + b + 255) / 256 * 256; return at; };
+        const size_t per_image = sizeof(int32_t) * (size_t)tiles * 32, words = sizeof(uint32_t) * (size_t)tiles;
+        const size_t at_ids0 = place(per_image), at_ids1 = place(per_image), at_slot = place(per_image), at_work_of = place(per_image);
+        const size_t at_mask = place(words), at_open = place(words), at_settled = place(words), at_working = place(words);
+        const size_t at_done = place(tiles), at_flag = place(kMarksOffset + (size_t)tiles);
+        CK(cudaMalloc(&c->per_tile, bytes));
+        CK(cudaMemsetAsync(c->per_tile, 0, bytes, c->stream));
+        unsigned char *const b = c->per_tile;
+        c->ids[0] = reinterpret_cast<int32_t *>(b + at_ids0);
+        c->ids[1] = reinterpret_cast<int32_t *>(b + at_ids1);
+        c->slot = reinterpret_cast<int32_t *>(b + at_slot);
+        c->work_of = reinterpret_cast<int32_t *>(b + at_work_of);
+        c->mask = reinterpret_cast<uint32_t *>(b + at_mask);
+        c->open_mask = reinterpret_cast<uint32_t *>(b + at_open);
+        c->settled = reinterpret_cast<uint32_t *>(b + at_settled);
+        c->working = reinterpret_cast<uint32_t *>(b + at_working);
+        c->tile_done = b + at_done;
+        c->in_flag = reinterpret_cast<int32_t *>(b + at_flag);
+        c->has_floats = b + at_flag + kMarksOffset;
+    }
     CK(cudaMalloc(&c->xw, sizeof(uint32_t) * (size_t)tiles * c->nw));
     CK(cudaMemsetAsync(c->xw, 0, sizeof(uint32_t) * (size_t)tiles * c->nw, c->stream));     // incl. the zero words behind the neurons
-    CK(cudaMalloc(&c->in_flag, kMarksOffset + (size_t)tiles));
-    CK(cudaMemsetAsync(c->in_flag, 0, kMarksOffset + (size_t)tiles, c->stream));
-    c->has_floats = reinterpret_cast<unsigned char *>(c->in_flag) + kMarksOffset;
     c->tiles_cap = tiles;
     return SPDNN_OK;
 }
@@ -1325,9 +1334,7 @@ int spdnn_create(spdnn_t **out, int device, int neurons, int layers, float bias,
     c->tile_stride = ((long long)neurons + 1) * 32;
     c->nw = front_words_per_tile(neurons);
     DeviceGuard guard(device);
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, device));
-    c->sm_count = prop.multiProcessorCount;
+    CK(cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device));      // (cudaGetDeviceProperties takes 3 ms)
     CK(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
     c->stream = c->own_stream;
     CK(cudaEventCreate(&c->ev_prep0)); CK(cudaEventCreate(&c->ev_prep1));
