@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -62,26 +63,32 @@ struct HostLayer {
     std::vector<int32_t> rows;     // [n][k] ascending input neuron per output neuron; padding = n
     std::vector<float> vals;       // [n][k]; padding 0
     uint64_t hash1 = 0, hash2 = 0; // content hashes (128 bits together)
+    // For keeps_top, found on the way through the columns: the fewest entries of one and, where weights differ, the least
+    // sum of clip * weight over a column (NaN where a sum is).
+    int least_entries = 0;
+    float least_sum = 0.0f;
 };
 
-// Returns an empty string on success, else the reason the layer is rejected.
-inline std::string canonicalize_layer(int n, const int32_t *col_ptr, const int32_t *row_idx, const float *val, HostLayer &out) {
+// Returns an empty string on success, else the reason the layer is rejected.  clip: see HostLayer::least_sum.
+inline std::string canonicalize_layer(int n, const int32_t *col_ptr, const int32_t *row_idx, const float *val, HostLayer &out,
+                                      float clip = 0.0f) {
     if (n <= 0 || n > (1 << 26)) return "neurons must be in [1, 2^26]";
     if (!col_ptr || !row_idx) return "col_ptr/row_idx is null";
     if (col_ptr[0] != 0) return "col_ptr[0] must be 0";
-    int kmax = 0;
+    int kmax = 0, kmin = 4096;
     for (int c = 0; c < n; ++c) {
         const int64_t cnt = (int64_t)col_ptr[c + 1] - col_ptr[c];
         if (cnt < 0) return "col_ptr must be non-decreasing";
         if (cnt > 4096) return "more than 4096 non-zeros in one column is not supported";
         kmax = std::max<int>(kmax, (int)cnt);
+        kmin = std::min<int>(kmin, (int)cnt);
     }
     const int64_t nnz = col_ptr[n];
     const int k = std::max(4, (kmax + 3) / 4 * 4);
     const float w0 = val ? (nnz ? val[0] : 0.0625f) : 0.0625f;
     bool uniform = is_pow2_float(w0);
     out = HostLayer();
-    out.n = n; out.k = k; out.nnz = nnz; out.w = w0;
+    out.n = n; out.k = k; out.nnz = nnz; out.w = w0; out.least_entries = kmin;
     // ascending row, stable for equal rows (repeated entries stay separate terms, as a COO with
     // repeated triplets would be summed)
     out.rows.assign((size_t)n * k, n);
@@ -92,15 +99,18 @@ inline std::string canonicalize_layer(int n, const int32_t *col_ptr, const int32
     for (int c = 0; c < n; ++c) {
         const int s = col_ptr[c], e = col_ptr[c + 1];
         tmp.clear();
+        bool ascending = true;
         for (int i = s; i < e; ++i) {
             const int32_t r = row_idx[i];
             if (r < 0 || r >= n) return "row index out of range in column " + std::to_string(c);
             const float v = val ? val[i] : 0.0625f;
             if (v != w0) uniform = false;
+            ascending &= tmp.empty() || tmp.back().first <= r;
             tmp.emplace_back(r, v);
         }
-        std::stable_sort(tmp.begin(), tmp.end(),
-                         [](const std::pair<int32_t, float> &a, const std::pair<int32_t, float> &b) { return a.first < b.first; });
+        if (!ascending)                            // (the usual column comes in order, and the sort allocates a buffer)
+            std::stable_sort(tmp.begin(), tmp.end(),
+                             [](const std::pair<int32_t, float> &a, const std::pair<int32_t, float> &b) { return a.first < b.first; });
         uint64_t h = 0x9E3779B97F4A7C15ull;
         for (size_t i = 0; i < tmp.size(); ++i) {
             out.rows[(size_t)c * k + i] = tmp[i].first;
@@ -112,34 +122,46 @@ inline std::string canonicalize_layer(int n, const int32_t *col_ptr, const int32
         h1 = mix64(h1 ^ h);
         h2 = mix64(h2 + h * 0x9E3779B97F4A7C15ull + (uint64_t)c);
     }
+    if (!uniform) {
+        // four columns at a time, whose chains of adds overlap; the product is rounded on its way from double, before it
+        // is added, as in the kernels
+        float least = std::numeric_limits<float>::infinity();
+        bool nan = false;
+        for (int c0 = 0; c0 < n; c0 += 4) {
+            const float *v[4];
+            int cnt[4];
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int q = 0; q < 4; ++q) {
+                const int c = std::min(c0 + q, n - 1);
+                v[q] = &out.vals[(size_t)c * k];
+                cnt[q] = col_ptr[c + 1] - col_ptr[c];
+            }
+            for (int i = 0; i < k; ++i)
+                for (int q = 0; q < 4; ++q) sum[q] += i < cnt[q] ? (float)((double)clip * (double)v[q][i]) : 0.0f;
+            for (int q = 0; q < 4; ++q) {
+                nan |= std::isnan(sum[q]);
+                least = std::min(least, sum[q]);
+            }
+        }
+        out.least_sum = nan ? std::numeric_limits<float>::quiet_NaN() : least;
+    }
     out.uniform = uniform;
     out.hash1 = h1; out.hash2 = h2;
     return std::string();
 }
 
-// Whether the layer maps the vector whose every entry is `clip` onto itself: each column's sum, added and rounded as the
-// kernels do it, reaches clip with the bias.  (Every product and sum is rounded to fp32 by its store.)
+// Whether the layer maps the vector whose every entry is `clip` (the one it was canonicalised with, > 0) onto itself: each
+// column's sum, added and rounded as the kernels do it, reaches clip with the bias.  The least sum decides, because
+// adding the bias does not reverse an order; with a uniform weight (added first, then scaled) that of the shortest column.
 inline bool keeps_top(const HostLayer &h, float bias, float clip) {
-    std::vector<signed char> of_count(h.k + 1, -1);      // uniform weight: the sum depends on the number of entries alone
-    for (int c = 0; c < h.n; ++c) {
-        const int32_t *r = &h.rows[(size_t)c * h.k];
-        int count = h.k;                                  // padding (rows past the last neuron) is at the end
-        while (count > 0 && r[count - 1] >= h.n) --count;
-        if (h.uniform && of_count[count] >= 0) {
-            if (!of_count[count]) return false;
-            continue;
-        }
-        volatile float sum = 0.0f;
-        for (int i = 0; i < count; ++i) {
-            volatile float term = h.uniform ? clip : clip * h.vals[(size_t)c * h.k + i];
-            sum = sum + term;
-        }
-        volatile float y = h.uniform ? sum * h.w : sum;
-        y = y + bias;
-        of_count[count] = y >= clip;
-        if (!(y >= clip)) return false;
+    float sum = h.least_sum;
+    if (h.uniform) {
+        sum = 0.0f;
+        for (int i = 0; i < h.least_entries; ++i) sum += clip;
+        volatile float scaled = sum * h.w;
+        sum = scaled;
     }
-    return true;
+    return sum + bias >= clip;
 }
 
 // Groups the columns of a layer whose (id sequence, weights) coincide.  ids == nullptr: the

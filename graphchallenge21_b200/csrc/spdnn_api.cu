@@ -1466,7 +1466,7 @@ int spdnn_set_layer_csc(spdnn_t *c, int layer, const int32_t *col_ptr, const int
     PerLayerTables p;
     std::string why;
     try {
-        why = canonicalize_layer(c->n, col_ptr, row_idx, val, *host);
+        why = canonicalize_layer(c->n, col_ptr, row_idx, val, *host, c->clip);
         if (!why.empty()) return fail(c, SPDNN_ERR_ARG, "layer %d: %s", layer, why.c_str());
         c->graph_dirty = true;
         // equal layers share one device copy

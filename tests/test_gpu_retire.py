@@ -69,3 +69,66 @@ def test_large_batches_retire_in_short_chunks(oracle):
         assert np.array_equal(g.layer_live(), want_l)
         assert np.array_equal(g.categories(), want_c)
         assert np.array_equal(g.activations(), want_a)
+
+
+def _column_value(clip, weights, bias, uniform):
+    """What a column of an all-clip input yields before it is cut off at clip, rounded step by step as the kernels do."""
+    s = np.float32(0)
+    for w in weights:
+        s = np.float32(s + (clip if uniform else np.float32(clip * w)))
+    if uniform:
+        s = np.float32(s * weights[0])
+    return np.float32(s + bias)
+
+
+@pytest.mark.parametrize("clip", [32.0, 2.5, 0.1])
+@pytest.mark.parametrize("kind", ["general", "uniform", "short", "empty"])
+def test_the_last_bit_decides_whether_a_layer_keeps_the_top(kind, clip, oracle):
+    """One column of one layer yields clip, or the number below it: all images are all clip until then."""
+    n, L, k, b = 64, 14, 16, 50
+    rng = np.random.default_rng(11)
+    clip = np.float32(clip)
+    rows = [np.sort(np.argpartition(rng.random((n, n)), k, axis=1)[:, :k], axis=1).astype(np.int32) for _ in range(L)]
+    vals = [rng.uniform(0.1, 0.2, (n, k)).astype(np.float32) for _ in range(L)]
+    uniform = kind != "general"
+    variants = []
+    if kind == "general":
+        bias = np.float32(-0.1 * clip)
+        w = vals[11][5]
+        w[:] = np.float32(0.06)                            # too little without the last one; the least last one that does
+        lo, hi = np.float32(0.0), np.float32(1.0)
+        while np.nextafter(lo, hi) < hi:
+            mid = np.float32((lo + hi) / 2)
+            if mid in (lo, hi):
+                break
+            w[-1] = mid
+            lo, hi = (lo, mid) if _column_value(clip, w, bias, False) >= clip else (mid, hi)
+        for last, keeps in ((hi, True), (lo, False)):
+            v = [x.copy() for x in vals]
+            v[11][5, -1] = last
+            assert (_column_value(clip, v[11][5], bias, False) >= clip) == keeps
+            variants.append((rows, v, bias, keeps))
+    else:
+        vals = [np.full((n, k), 0.0625, np.float32) for _ in range(L)]
+        below = np.float32(clip - np.nextafter(clip, np.float32(0)))
+        if kind == "uniform":                              # 16 times clip / 16, and too little bias to matter or enough
+            biases = [np.float32(f * below) for f in (0.0, -0.25, -0.75, -1.0, -3.0, -9.0)]
+            variants = [(rows, vals, x, bool(_column_value(clip, vals[0][0], x, True) >= clip)) for x in biases]
+            assert variants[0][3] and not variants[-1][3]
+        else:
+            short = [r.copy() for r in rows]
+            short[11][5, 15 if kind == "short" else 0:] = -1
+            variants = [(short, vals, np.float32(0), False), (rows, vals, np.float32(0), True)]
+    y0 = np.full((b, n), clip, np.float32)
+    for r, v, bias, keeps in variants:
+        layers = [(x, None if uniform else y) for x, y in zip(r, v)]
+        want_c, want_a, want_l = oracle.infer(y0, layers, float(bias), clip=float(clip))
+        with SpDNN(n, L, float(bias), clip=float(clip)) as g:
+            for l, (x, y) in enumerate(layers):
+                g.set_layer_rows(l, x, y)
+            g.set_input_dense(y0)
+            g.infer()
+            assert np.array_equal(g.layer_live(), want_l)
+            assert np.array_equal(g.categories(), want_c)
+            assert np.array_equal(g.activations(), want_a)
+            assert g.shortcuts()["retired_images"] == (b if keeps else 0)
