@@ -534,6 +534,8 @@ static __global__ void finalize_kernel(const LoopCtl *ctl0, int nsteps, const in
                                        uint32_t *working, const int32_t *first_id) {
     const LoopCtl c = ctl0[nsteps];
     const int t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    const int32_t code = *status;                // (on their way while the loops below run)
+    const uint32_t left_out = *skipped;
     int32_t *ids = c.ids_buf ? ids1 : ids0;
     const int32_t *from = c.ids_buf ? ids0 : ids1;
     for (int j = t; j < c.live; j += step) {
@@ -544,7 +546,10 @@ static __global__ void finalize_kernel(const LoopCtl *ctl0, int nsteps, const in
     }
     for (int q = t; q < layers; q += step) host.died_at[q] = died_at[q];
     for (int q = t; q <= nsteps; q += step) host.ctl[q] = ctl0[q];
-    if (t == 0) { *host.status = *status; *host.skipped = *skipped; }
+    if (t == 0) {
+        *host.status = code;
+        *host.skipped = left_out;
+    }
 }
 
 // dense_cell: where the first launch of a pass finds the caller's row-major input when that launch

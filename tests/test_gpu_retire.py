@@ -18,7 +18,7 @@ def run(n, layers, bias, clip, y0, first):
         for part in (y0, y0[: max(1, len(y0) // 3)]):          # a second, smaller batch in the same buffers
             g.set_input_dense(part, first)
             res = g.infer()
-            out.append((g.categories().copy(), g.activations(), g.layer_live().copy(), res.survivors))
+            out.append((g.categories().copy(), g.activations(), g.layer_live().copy(), res.survivors, g.shortcuts()["retired_images"]))
         return out
 
 
@@ -47,11 +47,16 @@ def test_retired_images_are_survivors(kind, n, b, L, env, monkeypatch, oracle):
         y0[:] = clip
         y0[::7] = 0.0
     got = run(n, layers, bias, clip, y0, 11)
-    for part, (cats, act, live, survivors) in zip((y0, y0[: max(1, b // 3)]), got):
+    for part, (cats, act, live, survivors, retired) in zip((y0, y0[: max(1, b // 3)]), got):
         wc, wa, wl = oracle.infer(part, layers, bias, clip=clip, first_image=11)
         assert np.array_equal(live, wl)
         assert np.array_equal(cats, wc) and survivors == len(wc)
         assert np.array_equal(act, wa)
+        assert retired <= (wa == clip).all(axis=1).sum()
+        if "SPDNN_RETIRE" in env:
+            assert retired == 0
+        elif n < 16384 and L >= 12 and kind in ("random", "general", "all"):
+            assert retired > 0
 
 
 def test_large_batches_retire_in_short_chunks(oracle):
