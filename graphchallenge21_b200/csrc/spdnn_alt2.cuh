@@ -320,9 +320,9 @@ alt2_kernel(const ResArgs a) {
                         // as many as the ring of word buffers can hold without overwriting the buffer they start from).  A
                         // period may take several groups, for a table copy can bring fewer layers than it has.
                         if (watch_left == 0 && careful == 0 && ring_periods > 0 && li >= a.period_from) {
-                            int len = first_watch ? a.period : ring_periods * a.period;
-                            if (li + len >= nl) len = a.period;
-                            if (li + len < nl) {
+                            const int room = (nl - 1 - li) / a.period;       // periods with a layer behind them
+                            const int len = min(first_watch ? 1 : ring_periods, room) * a.period;
+                            if (len > 0) {
                                 watch_left = len;
                                 watch_from = ws;
                                 first_watch = false;
